@@ -118,9 +118,20 @@ const SizeVariants* host_variants(int eng_slot) {
 constexpr int kMaxDevices = 64;
 DeviceState g_devices[kMaxDevices];
 
+// v * 2^62 as h*2^32 + l with l signed (|v| <= sqrt 2)
+void fxn_limbs(long double v, int* h, int* l) {
+  const long long q = llroundl(v * 4611686018427387904.0L);  // 2^62
+  *l = (int)(unsigned)q;
+  *h = (int)((q - *l) >> 32);
+}
+
+// Twiddle table of a plan in each engine's layout.  f64: (cos, -sin) pairs.
+// fx, 4 ints per entry: 30-bit limbs of both parts, or (d.natural) the natural
+// limbs of wr and of wi - wr; there, behind all entries, 2 ints per entry: the
+// limbs of -(wr + wi).
 void build_twiddles(const KernelDesc& d, std::vector<double>& f64, std::vector<int>& fx) {
   f64.assign((size_t)d.tw_entries * 2, 0.0);
-  fx.assign((size_t)d.tw_entries * 4, 0);
+  fx.assign((size_t)d.tw_entries * (d.natural ? 6 : 4), 0);
   int off = 0, p = d.radix[0];
   for (int s = 1; s < d.passes; ++s) {
     const int R = d.radix[s];
@@ -131,8 +142,15 @@ void build_twiddles(const KernelDesc& d, std::vector<double>& f64, std::vector<i
         const int e = off + (m - 1) * p + k;
         f64[2 * e] = (double)c;
         f64[2 * e + 1] = (double)(-sn);
-        fx_limbs(c, &fx[4 * e], &fx[4 * e + 1]);
-        fx_limbs(-sn, &fx[4 * e + 2], &fx[4 * e + 3]);
+        if (d.natural) {
+          int* sum = &fx[4 * (size_t)d.tw_entries + 2 * e];
+          fxn_limbs(c, &fx[4 * e], &fx[4 * e + 1]);
+          fxn_limbs(-sn - c, &fx[4 * e + 2], &fx[4 * e + 3]);
+          fxn_limbs(sn - c, &sum[0], &sum[1]);
+        } else {
+          fx_limbs(c, &fx[4 * e], &fx[4 * e + 1]);
+          fx_limbs(-sn, &fx[4 * e + 2], &fx[4 * e + 3]);
+        }
       }
     off += (R - 1) * p;
     p *= R;
@@ -174,7 +192,8 @@ void init_device(DeviceState& ds) {
         std::vector<double> f64;
         std::vector<int> fx;
         build_twiddles(d, f64, fx);
-        const size_t bytes = (size_t)(d.tw_entries > 0 ? d.tw_entries : 1) * 16;
+        const size_t used = eng == 0 ? f64.size() * sizeof(double) : fx.size() * sizeof(int);
+        const size_t bytes = used > 0 ? used : 16;
         void* p = nullptr;
         e = cudaMalloc(&p, bytes);
         if (e != cudaSuccess) {
@@ -184,7 +203,7 @@ void init_device(DeviceState& ds) {
           return;
         }
         const void* src = eng == 0 ? (const void*)f64.data() : (const void*)fx.data();
-        if (d.tw_entries > 0) e = cudaMemcpy(p, src, (size_t)d.tw_entries * 16, cudaMemcpyHostToDevice);
+        if (d.tw_entries > 0) e = cudaMemcpy(p, src, used, cudaMemcpyHostToDevice);
         if (e != cudaSuccess) {
           cudaGetLastError();
           ds.init_status = FFTOC_ERR_CUDA;

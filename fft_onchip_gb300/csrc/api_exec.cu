@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "../../include/fftoc.h"
+#include "fft_core.cuh"
 #include "internal.h"
 
 namespace fftoc {
@@ -39,6 +40,7 @@ extern "C" fftoc_status fftoc_exec_twiddles(int n, int engine, const int radix[4
     return set_error(FFTOC_ERR_UNSUPPORTED, "executors exist for the binary64 and fixed-point engines");
 
   KernelDesc d;
+  d.natural = n >= kNaturalMinN ? 1 : 0;
   long long prod = 1;
   bool tail = false;  // an unused pass (1) was seen: only 1s may follow
   for (int s = 0; s < 4; ++s) {
@@ -72,7 +74,7 @@ extern "C" fftoc_status fftoc_exec_twiddles(int n, int engine, const int radix[4
   std::vector<double> f64;
   std::vector<int> fx;
   twiddle_tables(d, f64, fx);
-  const size_t bytes = (size_t)d.tw_entries * 16;
+  const size_t bytes = eng == FFTOC_ENGINE_F64 ? f64.size() * sizeof(double) : fx.size() * sizeof(int);
   void* p = nullptr;
   if ((e = cudaMalloc(&p, bytes)) != cudaSuccess) {
     cudaGetLastError();

@@ -13,7 +13,7 @@
 // kNoAllocScratchBytes instead, keeps its twiddle tables and error flag in
 // file-scope __device__ arrays too, and runs H2D copy, transform and D2H copy
 // on the caller's stream.  The arrays are part of the loaded module: every GPU
-// that loads the library holds them (~35 MiB) until the process exits.
+// that loads the library holds them (~36 MiB) until the process exits.
 #include <atomic>
 #include <cstring>
 #include <mutex>
@@ -31,7 +31,7 @@ fftoc_status set_error(fftoc_status st, const std::string& msg);
 namespace {
 
 constexpr size_t kNoAllocScratchBytes = 32u << 20;  // largest batch*n*16 accepted
-constexpr int kNoAllocTwiddleEntries = 192 * 1024;   // 16-byte entries, every compiled plan of both engines
+constexpr int kNoAllocTwiddleEntries = 256 * 1024;   // 16-byte units, every compiled plan of both engines
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 __device__ __align__(256) int4 g_noalloc_twiddles[kNoAllocTwiddleEntries];
@@ -51,7 +51,7 @@ struct NoAllocDevice {
   int* err = nullptr;
   int sms = 0;
   SizeVariants var[2][kNumSizes];
-  int tw_offset[2][kNumSizes][kMaxVariants] = {};  // entry offset of each plan's table
+  int tw_offset[2][kNumSizes][kMaxVariants] = {};  // 16-byte offset of each plan's table
 };
 
 constexpr int kMaxDevices = 64;
@@ -90,17 +90,10 @@ void setup(NoAllocDevice& nd, int dev) {
         std::vector<int> fx;
         twiddle_tables(d, f64, fx);
         nd.tw_offset[slot][i][v] = (int)host.size();
-        for (int k = 0; k < d.tw_entries; ++k) {
-          int4 w;
-          if (slot == 0) {
-            const double re = f64[2 * k], im = f64[2 * k + 1];
-            memcpy(&w.x, &re, 8);
-            memcpy(&w.z, &im, 8);
-          } else {
-            w = make_int4(fx[4 * k], fx[4 * k + 1], fx[4 * k + 2], fx[4 * k + 3]);
-          }
-          host.push_back(w);
-        }
+        const size_t used = slot == 0 ? f64.size() * sizeof(double) : fx.size() * sizeof(int);
+        host.resize(host.size() + (used + 15) / 16);
+        if (used > 0)
+          memcpy(host.data() + nd.tw_offset[slot][i][v], slot == 0 ? (const void*)f64.data() : (const void*)fx.data(), used);
       }
     }
   if ((int)host.size() > kNoAllocTwiddleEntries) {

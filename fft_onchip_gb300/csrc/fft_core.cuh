@@ -15,8 +15,10 @@
 //   EngFx  — 64-bit block fixed point.  Each transform is scaled by a power of
 //            two taken from its largest exponent so that no value can overflow
 //            (headroom for the worst-case growth of N), adds are exact 64-bit
-//            integer adds, and products use 30-bit limbs on IMAD.WIDE.  The
-//            conversion back to binary64 rounds once (cvt.rn.f64.s64).
+//            integer adds, and products use 32 x 32 -> 64 multiplies: on 30-bit
+//            limbs for N <= 32 (EngFxT), on the natural 32-bit words from
+//            N = 64 up (EngFxN).  The conversion back to binary64 rounds once
+//            (cvt.rn.f64.s64).
 #pragma once
 #include <type_traits>
 #include <cstdint>
@@ -75,6 +77,7 @@ struct EngF64 {
   using TW = double2;   // (cos, -sin) of the twiddle
   struct KC { double c; };
   static constexpr int kId = 1;
+  static constexpr bool kNatural = false;
   FFTOC_HD static S add(S a, S b) { return a + b; }
   FFTOC_HD static S sub(S a, S b) { return a - b; }
   FFTOC_HD static S add3(S a, S b, S c) { return (a + b) + c; }
@@ -111,6 +114,7 @@ struct EngFxT {
   using TW = int4;      // (wr.h, wr.l, wi.h, wi.l): w*2^60 = h*2^30 + l, 0 <= l < 2^30
   using KC = FxKC;
   static constexpr int kId = 2;
+  static constexpr bool kNatural = false;
   FFTOC_HD static S add(S a, S b) { return a + b; }
   FFTOC_HD static S sub(S a, S b) { return a - b; }
   // Three-operand sums as one PTX sequence each: the front end cannot share
@@ -205,6 +209,100 @@ struct EngFxT {
 };
 using EngFx = EngFxT<false>;
 
+// Fixed point on the natural 32-bit words (transforms of N >= 64).  A value is
+// split as x = xh * 2^32 + xl with xl its low word read as signed, so a split
+// costs one instruction (the low word's sign carried into the high word).
+//
+// Twiddles are held as w * 2^62 = wh * 2^32 + wl, and a product takes three
+// real products instead of four:
+//   k1 = wr (xr + xi),  yr = k1 - xi (wr + wi),  yi = k1 + xr (wi - wr),
+// the sums and differences of w's parts from the table.  It comes at quarter
+// scale, x * w / 4, where the middle sum's high word is its share of the
+// result with no funnel shift, or at full scale for two more instructions a
+// component.  Transforms that have to give up low bits to the growth of N
+// anyway do so in their first passes with twiddles (FxPasses): the input is
+// converted at 53 bits for every N, and the last pass has at least the bits
+// that a conversion at the final scale from the start would leave.
+// The kernels are bound by the integer pipes.  Per warp and SM quadrant a
+// 32 x 32 -> 64 multiply takes four cycles of the FMA-heavy pipe and two of
+// the ALU (both measured by mixing it with ALU instructions), every other
+// integer instruction two cycles of one of them, so fewer and narrower
+// instructions are what counts: a product is 9 multiplies and about 9 others
+// at quarter scale, against 12 and about 17 with the 30-bit limbs of EngFxT
+// (hardware counters over a kernel of products alone: 18.7 against 29).
+// With the slots and exponent range of fft_kernel.cuh, 1 GiB of input, on one
+// GB300: N = 512 430 -> 371 us (5.0 -> 5.8 TB/s), N = 4096 626 -> 576 us,
+// N = 1024 (82 MB) 47.1 -> 41.0 us.
+struct EngFxN {
+  using S = long long;
+  using TW = int4;  // limbs (h, l) of wr and of wi - wr; those of -(wr + wi) in an int2 table behind
+  static constexpr int kId = 2;
+  static constexpr bool kNatural = true;
+  FFTOC_HD static S add(S a, S b) { return a + b; }
+  FFTOC_HD static S sub(S a, S b) { return a - b; }
+  FFTOC_HD static S add3(S a, S b, S c) { return EngFx::add3(a, b, c); }
+  FFTOC_HD static S addsub(S a, S b, S c) { return EngFx::addsub(a, b, c); }
+  FFTOC_HD static S subadd(S a, S b, S c) { return EngFx::subadd(a, b, c); }
+  FFTOC_HD static S sub3(S a, S b, S c) { return EngFx::sub3(a, b, c); }
+  FFTOC_HD static void split(S x, int& xh, int& xl) {
+    xl = (int)(unsigned)x;
+    xh = (int)((unsigned long long)x >> 32) + (int)((unsigned)x >> 31);
+  }
+  // a * b, 32 x 32 -> 64.  Sums of products are written as plain 64-bit
+  // additions of these: the assembler then fuses each addition into a
+  // multiply-add where that is cheaper.  Spelled out as mad.wide chains the
+  // same product took 25 instructions instead of 19.
+  FFTOC_HD static S mul(int a, int b) { return EngFx::mulw(a, b); }
+  // x * w, or x * w / 4 (QUARTER); |xr + j xi| <= 2^61.5: the middle sums stay
+  // below (sqrt(5) + 1 + sqrt(1/2)) * 2^61 < 2^63.
+  template <bool QUARTER>
+  FFTOC_HD static void cmul(S& xr, S& xi, const int4 w, const int2 c) {
+    int rh, rl, ih, il, sh, sl;
+    split(xr, rh, rl);
+    split(xi, ih, il);
+    split(xr + xi, sh, sl);
+    const S m = mul(sl, w.x) + mul(sh, w.y), h = mul(sh, w.x);
+    const S mr = mul(il, c.x) + mul(ih, c.y) + m;
+    const S mi = mul(rl, w.z) + mul(rh, w.w) + m;
+    const S hr = mul(ih, c.x) + h, hi = mul(rh, w.z) + h;
+    if constexpr (QUARTER) {
+      xr = hr + (mr >> 32);
+      xi = hi + (mi >> 32);
+    } else {
+      xr = (S)((unsigned long long)hr << 2) + (mr >> 30);
+      xi = (S)((unsigned long long)hi << 2) + (mi >> 30);
+    }
+  }
+  // x * sqrt(1/2) = x + x * (sqrt(1/2) - 1), full scale
+  FFTOC_HD static S mulh(S x) {
+    constexpr FxKC V = {-1257966796, -102865788};
+    int xh, xl;
+    split(x, xh, xl);
+    const S m = mul(xl, V.h) + mul(xh, V.l);
+    return mul(xh, V.h) + x + (m >> 32);
+  }
+  // (r, i) -> (c r + s i, c i - s r), c = cos(pi/8), s = sin(pi/8), full scale:
+  // with t = s (r + i), c r + s i = r + (t + (c - s - 1) r) and
+  // c i - s r = i - (t + (1 - c - s) i); constants v as v * 2^64 = h * 2^32 + l,
+  // l signed.  |r + j i| <= 2^59.5 keeps the middle sums below 2^63.
+  FFTOC_HD static void rot8(S& r, S& i) {
+    constexpr FxKC S8 = {1643612827, -1163556025}, E = {-1970547745, -641423873}, F = {-1316677908, -1326431372};
+    int rh, rl, ih, il, sh, sl;
+    split(r, rh, rl);
+    split(i, ih, il);
+    split(r + i, sh, sl);
+    const S m = mul(sl, S8.h) + mul(sh, S8.l), h = mul(sh, S8.h);
+    const S mr = mul(rl, E.h) + mul(rh, E.l) + m;
+    const S mi = mul(il, F.h) + mul(ih, F.l) + m;
+    r = r + mul(rh, E.h) + h + (mr >> 32);
+    i = i - (mul(ih, F.h) + h + (mi >> 32));
+  }
+};
+
+// Smallest N on the natural words; below it the kernels stream at the HBM
+// rate (EngFxT) and their register budgets are full.
+constexpr int kNaturalMinN = 64;
+
 // constants of the DFT kernels, per engine
 template <class E> struct Konst;
 template <> struct Konst<EngF64> {
@@ -279,7 +377,10 @@ struct UnevenDefault : PL {
 // The engine a plan's kernels compute with: the fixed-point engine in the
 // plan's split form, or E unchanged.
 template <class E, class PL>
-using PlanEngine = typename std::conditional<E::kId == EngFx::kId && PL::IMAD_SPLIT, EngFxT<true>, E>::type;
+using PlanEngine = typename std::conditional<
+    E::kId != EngFx::kId, E,
+    typename std::conditional<(PL::N >= kNaturalMinN), EngFxN,
+                              typename std::conditional<PL::IMAD_SPLIT, EngFxT<true>, E>::type>::type>::type;
 
 // ---------------------------------------------------------------------------
 // Small forward DFTs on registers.  re[i], im[i] at compile-time indices
@@ -409,9 +510,135 @@ FFTOC_HD void dft16(typename E::S (&re)[PP], typename E::S (&im)[PP]) {
   for (int k = 0; k < 16; ++k) { re[B + k * ST] = xr[k]; im[B + k * ST] = xi[k]; }
 }
 
+// The 4-, 8- and 16-point DFTs of EngFxN.  The factors -i and -1 are folded
+// into the signs of the sums; the constant products are mulh and rot8.
+//
+// 4-point DFT of (x0, x1, x2, x3) with x2 replaced by -i x2 (MI2), x3 by -i x3
+// (MI3) or by -x3 (NEG3), outputs to y0..y3.
+template <bool MI2, bool MI3, bool NEG3, class S>
+FFTOC_HD void fxn_dft4(S x0r, S x0i, S x1r, S x1i, S x2r, S x2i, S x3r, S x3i, S& y0r, S& y0i, S& y1r, S& y1i, S& y2r,
+                       S& y2i, S& y3r, S& y3i) {
+  S tr, ti, ur, ui;  // x1 + x3, x1 - x3
+  if constexpr (MI3) {
+    tr = x1r + x3i; ti = x1i - x3r; ur = x1r - x3i; ui = x1i + x3r;
+  } else if constexpr (NEG3) {
+    tr = x1r - x3r; ti = x1i - x3i; ur = x1r + x3r; ui = x1i + x3i;
+  } else {
+    tr = x1r + x3r; ti = x1i + x3i; ur = x1r - x3r; ui = x1i - x3i;
+  }
+#ifdef FXN_3OP
+  using E = EngFxN;
+  if constexpr (MI2) {
+    y0r = E::add3(x0r, x2i, tr); y0i = E::subadd(x0i, x2r, ti);
+    y2r = E::addsub(x0r, x2i, tr); y2i = E::sub3(x0i, x2r, ti);
+    y1r = E::subadd(x0r, x2i, ui); y1i = E::addsub(x0i, x2r, ur);
+    y3r = E::sub3(x0r, x2i, ui); y3i = E::add3(x0i, x2r, ur);
+  } else {
+    y0r = E::add3(x0r, x2r, tr); y0i = E::add3(x0i, x2i, ti);
+    y2r = E::addsub(x0r, x2r, tr); y2i = E::addsub(x0i, x2i, ti);
+    y1r = E::subadd(x0r, x2r, ui); y1i = E::sub3(x0i, x2i, ur);
+    y3r = E::sub3(x0r, x2r, ui); y3i = E::subadd(x0i, x2i, ur);
+  }
+#else
+  S pr, pi, qr, qi;  // x0 + x2, x0 - x2
+  if constexpr (MI2) {
+    pr = x0r + x2i; pi = x0i - x2r; qr = x0r - x2i; qi = x0i + x2r;
+  } else {
+    pr = x0r + x2r; pi = x0i + x2i; qr = x0r - x2r; qi = x0i - x2i;
+  }
+  y0r = pr + tr; y0i = pi + ti;
+  y2r = pr - tr; y2i = pi - ti;
+  y1r = qr + ui; y1i = qi - ur;
+  y3r = qr - ui; y3i = qi + ur;
+#endif
+}
+
+template <bool MI2, bool MI3, bool NEG3, int B, int ST, int PP>
+FFTOC_HD void fxn_dft4_at(long long (&re)[PP], long long (&im)[PP]) {
+  fxn_dft4<MI2, MI3, NEG3>(re[B], im[B], re[B + ST], im[B + ST], re[B + 2 * ST], im[B + 2 * ST], re[B + 3 * ST],
+                           im[B + 3 * ST], re[B], im[B], re[B + ST], im[B + ST], re[B + 2 * ST], im[B + 2 * ST],
+                           re[B + 3 * ST], im[B + 3 * ST]);
+}
+
+// Sums and differences of x_m and x_{m+4}; W8 = (1 - i)/sqrt2 and W8^3 = -i W8
+// on the odd half, whose inputs 2 and 3 then carry a factor -i each.
+template <int B, int ST, int PP>
+FFTOC_HD void fxn_dft8(long long (&re)[PP], long long (&im)[PP]) {
+  using S = long long;
+  S ar[4], ai[4], br[4], bi[4];
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    ar[m] = re[B + m * ST] + re[B + (m + 4) * ST];
+    ai[m] = im[B + m * ST] + im[B + (m + 4) * ST];
+    br[m] = re[B + m * ST] - re[B + (m + 4) * ST];
+    bi[m] = im[B + m * ST] - im[B + (m + 4) * ST];
+  }
+  const S b1r = EngFxN::mulh(br[1] + bi[1]), b1i = EngFxN::mulh(bi[1] - br[1]);
+  const S b3r = EngFxN::mulh(br[3] + bi[3]), b3i = EngFxN::mulh(bi[3] - br[3]);
+  fxn_dft4<false, false, false>(ar[0], ai[0], ar[1], ai[1], ar[2], ai[2], ar[3], ai[3], re[B], im[B], re[B + 2 * ST],
+                                im[B + 2 * ST], re[B + 4 * ST], im[B + 4 * ST], re[B + 6 * ST], im[B + 6 * ST]);
+  fxn_dft4<true, true, false>(br[0], bi[0], b1r, b1i, br[2], bi[2], b3r, b3i, re[B + ST], im[B + ST], re[B + 3 * ST],
+                              im[B + 3 * ST], re[B + 5 * ST], im[B + 5 * ST], re[B + 7 * ST], im[B + 7 * ST]);
+}
+
+// dft16's 4 x 4 form.  Of the factors W16^(n2 k1): W^1 = rot8; W^2 = (1 - i)/sqrt2;
+// W^3 (r, i) = (p, -q) with (p, q) = rot8(i, r); W^4 = -i; W^6 = -i W^2; W^9 = -W^1.
+template <int B, int ST, int PP>
+FFTOC_HD void fxn_dft16(long long (&re)[PP], long long (&im)[PP]) {
+  using S = long long;
+  fxn_dft4_at<false, false, false, B, 4 * ST, PP>(re, im);
+  fxn_dft4_at<false, false, false, B + ST, 4 * ST, PP>(re, im);
+  fxn_dft4_at<false, false, false, B + 2 * ST, 4 * ST, PP>(re, im);
+  fxn_dft4_at<false, false, false, B + 3 * ST, 4 * ST, PP>(re, im);
+  // y[n2][k1] at B + (n2 + 4 k1) ST
+  auto at = [](int n2, int k1) { return B + (n2 + 4 * k1) * ST; };
+  auto w1 = [&](int i) {
+    S r = re[i], q = im[i];
+    EngFxN::rot8(r, q);
+    re[i] = r;
+    im[i] = q;
+  };
+  auto w2 = [&](int i) {
+    const S r = re[i], q = im[i];
+    re[i] = EngFxN::mulh(r + q);
+    im[i] = EngFxN::mulh(q - r);
+  };
+  auto w3 = [&](int i) {
+    S q = im[i], r = re[i];
+    EngFxN::rot8(q, r);
+    re[i] = q;
+    im[i] = -r;
+  };
+  w1(at(1, 1));
+  w2(at(2, 1));
+  w3(at(3, 1));
+  w2(at(1, 2));
+  w2(at(3, 2));  // times -i below; (2, 2) too
+  w3(at(1, 3));
+  w2(at(2, 3));  // times -i below
+  w1(at(3, 3));  // times -1 below
+  fxn_dft4_at<false, false, false, B, ST, PP>(re, im);
+  fxn_dft4_at<false, false, false, B + 4 * ST, ST, PP>(re, im);
+  fxn_dft4_at<true, true, false, B + 8 * ST, ST, PP>(re, im);
+  fxn_dft4_at<true, false, true, B + 12 * ST, ST, PP>(re, im);
+  S xr[16], xi[16];
+#pragma unroll
+  for (int k1 = 0; k1 < 4; ++k1)
+#pragma unroll
+    for (int k2 = 0; k2 < 4; ++k2) {
+      xr[k1 + 4 * k2] = re[B + (4 * k1 + k2) * ST];
+      xi[k1 + 4 * k2] = im[B + (4 * k1 + k2) * ST];
+    }
+#pragma unroll
+  for (int k = 0; k < 16; ++k) { re[B + k * ST] = xr[k]; im[B + k * ST] = xi[k]; }
+}
+
 template <class E, int R, int B, int ST, int PP>
 FFTOC_HD void dft(typename E::S (&re)[PP], typename E::S (&im)[PP]) {
-  if constexpr (R == 2) dft2<E, B, ST, PP>(re, im);
+  if constexpr (E::kNatural && R == 4) fxn_dft4_at<false, false, false, B, ST, PP>(re, im);
+  else if constexpr (E::kNatural && R == 8) fxn_dft8<B, ST, PP>(re, im);
+  else if constexpr (E::kNatural && R == 16) fxn_dft16<B, ST, PP>(re, im);
+  else if constexpr (R == 2) dft2<E, B, ST, PP>(re, im);
   else if constexpr (R == 4) dft4<E, B, ST, PP>(re, im);
   else if constexpr (R == 8) dft8<E, B, ST, PP>(re, im);
   else if constexpr (R == 16) dft16<E, B, ST, PP>(re, im);

@@ -15,6 +15,17 @@ template <int N> struct FxBits {
   static constexpr int B = (61 - ilog2c(N)) < 53 ? (61 - ilog2c(N)) : 53;
 };
 
+// Natural-word engine (EngFxN): the input has 53 bits, and passes 1..quarter
+// scale their products by a quarter, so that the last pass has 53 - 2 quarter
+// bits, at least FxBits<N>::B.  With input components below 2^53 the modulus
+// is below 2^53.5, times the radix of each pass and a quarter in those passes:
+// below 2^62.5 at the end for every N, and for every compiled plan at most
+// 2^61.5 at the input of a pass with twiddles and 2^59.5 at a radix-16 pass's
+// constant products.
+template <int N> struct FxPasses {
+  static constexpr int quarter = (53 - FxBits<N>::B) / 2;  // 0 up to N = 512, 1 at 1024 and 2048, 2 at 4096
+};
+
 // Rounding of the binary64 -> fixed-point input conversion of a size N.
 // Small transforms (N <= 32) stream at the HBM limit with every resident CTA
 // slot in use; there the truncating sequence (round toward zero, a negation
@@ -115,17 +126,24 @@ struct FxScale {
   int eref, K, kshift;
   bool slow, special;
 };
-template <int B>
+// H: bits of scale that the passes take off (EngFxN's quarter-scale products).
+template <int B, int H = 0>
 FFTOC_HD FxScale fx_scale(int em) {
   FxScale s;
   s.special = (em == 0x7FF);
   // subnormals (exponent field 0) are scaled like exponent field 1
   if (em < 1) em = 1;
-  s.K = em - 1022 - B;
+  s.K = em - 1022 - (B - H);
   s.kshift = (int)((unsigned)s.K << 20);
-  s.slow = (em < B) || (em > 1983 + B);
+  s.slow = (em < B - H) || (em > 1983 + (B - H));
   s.eref = em + 53 - B;
   return s;
+}
+// Scale of a size under engine E: input bits and the bits its passes take off.
+template <class E, int N>
+FFTOC_HD FxScale fx_size_scale(int em) {
+  if constexpr (E::kNatural) return fx_scale<53, 2 * FxPasses<N>::quarter>(em);
+  else return fx_scale<FxBits<N>::B>(em);
 }
 
 // Fast conversion for values within 2^31 of the transform's largest exponent
@@ -187,6 +205,23 @@ FFTOC_HD void fx_exponent_range(const double2 (&raw)[P], int& emax, int& emin) {
     emax = em;
     emin = en;
   } else {
+#ifdef __CUDA_ARCH__
+    // The sign-cleared words ordered as binary32 values (three-operand
+    // minimum and maximum with the sign cleared in the operand: 2.2
+    // instructions a point against 4.5 for the integer form).  Exponent
+    // fields from 0x7F8 up look like infinities and NaNs there: the maximum
+    // then is NaN or infinity, and the integer form below decides.
+    float fmax = 0.0f, fmin = __uint_as_float(0x7F800000u);
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      const float a = fabsf(__uint_as_float(hi_word(raw[i].x))), b = fabsf(__uint_as_float(hi_word(raw[i].y)));
+      asm("max.NaN.f32 %0, %0, %1, %2;" : "+f"(fmax) : "f"(a), "f"(b));
+      asm("min.f32 %0, %0, %1, %2;" : "+f"(fmin) : "f"(a), "f"(b));
+    }
+    emax = (int)(__float_as_uint(fmax) >> 20);
+    emin = (int)(__float_as_uint(fmin) >> 20);
+    if (emax < 0x7F8) return;
+#endif
     unsigned amax = 0u, amin = 0x7FFFFFFFu;
 #pragma unroll
     for (int i = 0; i < P; ++i) {
@@ -295,10 +330,22 @@ struct Fft {
       const int tp = t + T * b;
       const int k = tp & (p - 1);
       const TW* base = tw + PL::tw_offset(s) + k;
+      if constexpr (E::kNatural) {
+        const int2* sums = reinterpret_cast<const int2*>(tw + PL::TW_COUNT) + PL::tw_offset(s) + k;
+        constexpr bool QUARTER = s <= FxPasses<N>::quarter;
+        if constexpr (QUARTER) {  // the untwiddled input too
+          re[b] >>= 2;
+          im[b] >>= 2;
+        }
 #pragma unroll
-      for (int m = 1; m < R; ++m) {
-        const TW w = __ldg(base + (m - 1) * p);
-        E::cmul(re[b + B * m], im[b + B * m], w);
+        for (int m = 1; m < R; ++m)
+          E::template cmul<QUARTER>(re[b + B * m], im[b + B * m], __ldg(base + (m - 1) * p), __ldg(sums + (m - 1) * p));
+      } else {
+#pragma unroll
+        for (int m = 1; m < R; ++m) {
+          const TW w = __ldg(base + (m - 1) * p);
+          E::cmul(re[b + B * m], im[b + B * m], w);
+        }
       }
     }
     dft<E, R, b, B, P>(re, im);
@@ -320,25 +367,49 @@ struct Fft {
     return (tp - k) * R + k + m * p;
   }
 
+  // Slots and elements below are a base per thread and butterfly plus a
+  // constant per point.  The base's pad is computed once, since every constant
+  // is a multiple of 2^SH (left to the compiler, the pad of each slot cost
+  // 3 instructions a point and exchange at N = 512).
+  //
+  // slot of output 0 of butterfly b in pass s; output m is m * slot_step<s>() further
+  template <int s>
+  __device__ __forceinline__ static int slot0(int j, int t, int b) {
+    const int e = dest<s>(t, b, 0);
+    return j * NP + e + (e >> SH);
+  }
+  template <int s>
+  __host__ __device__ static constexpr int slot_step() {
+    constexpr int p = PL::span(s);
+    static_assert((s == 0 && PL::R[0] <= (1 << SH)) || p % (1 << SH) == 0, "an output's pad is a constant");
+    return p + (p >> SH);
+  }
+  static constexpr bool FIXED_PADS = PL::R[0] == (1 << SH);
+
   template <int s>
   __device__ __forceinline__ static void write_smem(S (&re)[P], S (&im)[P], int j, int t, longlong2* sm) {
     constexpr int R = PL::R[s];
     constexpr int B = P / R;
 #pragma unroll
-    for (int b = 0; b < B; ++b)
+    for (int b = 0; b < B; ++b) {
+      const int q = FIXED_PADS ? slot0<s>(j, t, b) : 0;
 #pragma unroll
       for (int m = 0; m < R; ++m) {
         longlong2 v;
         v.x = to_bits(re[b + B * m]);
         v.y = to_bits(im[b + B * m]);
-        sm[slot(j, dest<s>(t, b, m))] = v;
+        if constexpr (FIXED_PADS) sm[q + m * slot_step<s>()] = v;
+        else sm[slot(j, dest<s>(t, b, m))] = v;
       }
+    }
   }
 
   __device__ __forceinline__ static void read_smem(S (&re)[P], S (&im)[P], int j, int t, const longlong2* sm) {
+    constexpr bool fixed = T % (1 << SH) == 0 || (1 << SH) % T == 0;
+    const int q = j * NP + t + (t >> SH);
 #pragma unroll
     for (int i = 0; i < P; ++i) {
-      const longlong2 v = sm[slot(j, t + T * i)];
+      const longlong2 v = fixed ? sm[q + T * i + (T * i >> SH)] : sm[slot(j, t + T * i)];
       re[i] = from_bits(v.x);
       im[i] = from_bits(v.y);
     }
@@ -460,9 +531,11 @@ __device__ __forceinline__ void fft_tile(const Tile& tl, const typename E::TW* _
       raw[i] = make_double2(__longlong_as_double(v.x), __longlong_as_double(v.y));
     }
   } else {
-    const double2* src = tl.in_of(j) + t;  // in range or unused: loads are guarded
+    // RegTile's threads past the tile hold the offset of a transform of the tile
+    const double2* src = tl.in_of(j) + t;
 #pragma unroll
-    for (int i = 0; i < P; ++i) raw[i] = active ? Tile::load(src + T * i) : make_double2(0.0, 0.0);
+    for (int i = 0; i < P; ++i)
+      raw[i] = EK::kNatural || active ? Tile::load(src + T * i) : make_double2(0.0, 0.0);
   }
 
   S re[P], im[P];
@@ -477,7 +550,7 @@ __device__ __forceinline__ void fft_tile(const Tile& tl, const typename E::TW* _
     int em, emin;
     fx_exponent_range<P, TR>(raw, em, emin);
     em = fx_transform_max<T, TPB>(em, tid, j, reinterpret_cast<int*>(smem_raw + TPB * F::NP * 16));
-    const FxScale sc = fx_scale<FxBits<N>::B>(em);
+    const FxScale sc = fx_size_scale<EK, N>(em);
     special = sc.special;
     K = sc.K;
     kshift = sc.kshift;
@@ -561,9 +634,11 @@ __device__ __forceinline__ void fft_tile(const Tile& tl, const typename E::TW* _
             dst[F::template dest<NS - 1>(t, b, m)] = stored(b + BL * m);
       } else if (!redo) {
 #pragma unroll
-        for (int b = 0; b < BL; ++b)
+        for (int b = 0; b < BL; ++b) {
+          double2* q = dst + F::template dest<NS - 1>(t, b, 0);
 #pragma unroll
-          for (int m = 0; m < RL; ++m) dst[F::template dest<NS - 1>(t, b, m)] = value(b + BL * m);
+          for (int m = 0; m < RL; ++m) q[m * PL::span(NS - 1)] = value(b + BL * m);
+        }
       } else {
 #pragma unroll
         for (int b = 0; b < BL; ++b)
@@ -623,7 +698,7 @@ fft_fwd_kernel(const double2* __restrict__ in, double2* __restrict__ out, long l
   const int t = tid - j * T;
   const long long tile0 = (long long)blockIdx.x * TPB;
   const long long tr = tile0 + j;
-  const bool active = tr < batch;
+  const bool active = TPB == 1 || tr < batch;  // the grid has one CTA per tile
   const long long tile_elems = (min((long long)TPB, batch - tile0)) * N;
 
   // ---- load raw binary64 points: point i of this thread is element t + T*i
@@ -642,9 +717,17 @@ fft_fwd_kernel(const double2* __restrict__ in, double2* __restrict__ out, long l
       raw[i] = make_double2(__longlong_as_double(v.x), __longlong_as_double(v.y));
     }
   } else {
-    const double2* src = in + tr * N + t;
+    if constexpr (EK::kNatural) {
+      // threads past the batch load its last transform: no zero fill for
+      // predicated loads (2 instructions a point)
+      const double2* src = in + (TPB == 1 || active ? tr : batch - 1) * N + t;
 #pragma unroll
-    for (int i = 0; i < P; ++i) raw[i] = active ? __ldg(src + T * i) : make_double2(0.0, 0.0);
+      for (int i = 0; i < P; ++i) raw[i] = __ldg(src + T * i);
+    } else {
+      const double2* src = in + tr * N + t;
+#pragma unroll
+      for (int i = 0; i < P; ++i) raw[i] = active ? __ldg(src + T * i) : make_double2(0.0, 0.0);
+    }
   }
 
   S re[P], im[P];
@@ -659,7 +742,7 @@ fft_fwd_kernel(const double2* __restrict__ in, double2* __restrict__ out, long l
     int em, emin;
     fx_exponent_range<P, TR>(raw, em, emin);
     em = fx_transform_max<T, TPB>(em, tid, j, reinterpret_cast<int*>(smem_raw + TPB * F::NP * 16));
-    const FxScale sc = fx_scale<FxBits<N>::B>(em);
+    const FxScale sc = fx_size_scale<EK, N>(em);
     special = sc.special;
     K = sc.K;
     kshift = sc.kshift;
@@ -744,9 +827,11 @@ fft_fwd_kernel(const double2* __restrict__ in, double2* __restrict__ out, long l
             dst[F::template dest<NS - 1>(t, b, m)] = stored(b + BL * m);
       } else if (!redo) {
 #pragma unroll
-        for (int b = 0; b < BL; ++b)
+        for (int b = 0; b < BL; ++b) {
+          double2* q = dst + F::template dest<NS - 1>(t, b, 0);
 #pragma unroll
-          for (int m = 0; m < RL; ++m) dst[F::template dest<NS - 1>(t, b, m)] = value(b + BL * m);
+          for (int m = 0; m < RL; ++m) q[m * PL::span(NS - 1)] = value(b + BL * m);
+        }
       } else {
 #pragma unroll
         for (int b = 0; b < BL; ++b)

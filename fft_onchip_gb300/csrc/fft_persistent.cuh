@@ -76,9 +76,10 @@ template <class E, class PL, int NSTAGE>
 __global__ void __launch_bounds__(Fft<E, PL>::THREADS, PL::MINB)
 fft_fwd_persistent(const double2* __restrict__ in, double2* __restrict__ out, long long batch,
                    const typename E::TW* __restrict__ tw, int* __restrict__ err) {
-  using F = Fft<E, PL>;
+  using EK = PlanEngine<E, PL>;
+  using F = Fft<EK, PL>;
   using C = Persist<E, PL, NSTAGE>;
-  using S = typename E::S;
+  using S = typename EK::S;
   constexpr int N = PL::N, TPB = PL::TPB, P = PL::P, T = PL::T, NS = PL::S;
   extern __shared__ __align__(128) unsigned char smem_persist[];
   unsigned char* smem_raw = smem_persist;
@@ -161,7 +162,7 @@ fft_fwd_persistent(const double2* __restrict__ in, double2* __restrict__ out, lo
       int em, emin;
       fx_exponent_range<P, TR>(raw, em, emin);
       em = fx_transform_max<T, TPB>(em, tid, j, red);
-      const FxScale sc = fx_scale<FxBits<N>::B>(em);
+      const FxScale sc = fx_size_scale<EK, N>(em);
       special = sc.special;
       K = sc.K;
       kshift = sc.kshift;

@@ -241,7 +241,9 @@ fft_uneven_kernel(const UnevenArgs* __restrict__ a, int bin, const typename E::T
                      : "memory");
     }
     if constexpr (!FK::STAGED) {
-      const RegTile tl{a->in, a->out, ring[s0 * TPB + tid / FK::T], tile0, count};
+      // threads past the bucket take the tile's last transform (they store nothing)
+      const int last = count - tile0 < TPB ? (int)(count - tile0) - 1 : TPB - 1;
+      const RegTile tl{a->in, a->out, ring[s0 * TPB + min(tid / FK::T, last)], tile0, count};
       fft_tile<E, PL>(tl, tw, smem_raw);
     } else {
       const IndexedTile tl{a->in, a->out, ring + s0 * TPB, tile0, count};

@@ -28,7 +28,8 @@ struct KernelDesc {
   int ppt = 0;               // points per thread
   int passes = 0;
   int radix[4] = {1, 1, 1, 1};
-  int tw_entries = 0;        // twiddle table entries (16 bytes each)
+  int tw_entries = 0;        // twiddle table entries
+  int natural = 0;           // 1: fixed-point table in the natural-word layout (EngFxN)
   int persistent = 0;        // 1: grid-stride persistent CTAs with TMA prefetch (extra error-flag argument)
   int stages = 0;            // shared-memory stages of the persistent kernel
   int blocks_per_sm = 0;     // resident CTAs per SM (filled at device set-up)
@@ -132,7 +133,7 @@ fftoc_status dmma_plan_info(int n, fftoc_plan_info* info);
 fftoc_status launch_dmma(int n, const double* in, double* out, int64_t batch, cudaStream_t stream);
 
 // api.cu accessors: compiled plans per engine slot (0 F64, 1 FX), twiddle
-// tables of a plan (16 bytes per entry: double2 / 4 x int32 limbs), the plan
+// tables of a plan (double2, or int32 limbs: build_twiddles), the plan
 // currently chosen for (slot, size index), AUTO resolution, and the
 // per-thread error message.
 const SizeVariants* compiled_variants(int eng_slot);

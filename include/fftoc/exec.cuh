@@ -84,7 +84,8 @@ struct fft {
   static constexpr const char* print_type = Engine == FFTOC_ENGINE_F64 ? "fftoc_f64" : "fftoc_fx";
 
   using PL = typename plan_of<Size, transforms_per_block>::type;
-  using F = Fft<E, PL>;
+  using EK = PlanEngine<E, PL>;  // the arithmetic of the size's plans
+  using F = Fft<EK, PL>;
   static constexpr int NS = PL::S;
   static constexpr int kSlot = size_slot(Size);
   static_assert(T * transforms_per_block == max_threads_per_block, "every thread owns P points of one transform");
@@ -120,7 +121,7 @@ struct fft {
       int em, emin;
       fx_exponent_range<P, TR>(raw, em, emin);
       em = fx_transform_max<T, transforms_per_block>(em, tid, j, red);
-      const FxScale sc = fx_scale<FxBits<Size>::B>(em);
+      const FxScale sc = fx_size_scale<EK, Size>(em);
       special = sc.special;
       K = sc.K;
       kshift = sc.kshift;
