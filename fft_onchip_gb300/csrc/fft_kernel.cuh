@@ -298,6 +298,21 @@ __device__ __forceinline__ int fx_transform_max(int em, int tid, int j, int* red
   return em;
 }
 
+// Programmatic dependent launch (launch_plan): a kernel may start while the one
+// before it in its stream drains.  after_previous() waits for that kernel's
+// completion and must come before any access to the caller's buffers;
+// allow_next() lets the next kernel's CTAs take the places that this grid no
+// longer needs (they wait at their own after_previous()).
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// A point of the caller's input.  Not __ldg: the compiler takes read-only loads
+// as constant for the whole kernel and may move them above after_previous().
+__device__ __forceinline__ double2 load_point(const double2* p) {
+  double2 v;
+  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
+
 // --- the kernel ---------------------------------------------------------------
 template <class E, class PL>
 struct Fft {
@@ -673,6 +688,8 @@ fft_fwd_kernel(const double2* __restrict__ in, double2* __restrict__ out, long l
   extern __shared__ __align__(16) unsigned char smem_raw[];
   longlong2* sm = reinterpret_cast<longlong2*>(smem_raw);
 
+  allow_next();
+  after_previous();
   if constexpr (PL::PREFETCH) {
     if (threadIdx.x == 0 && batch * (PL::N * 16) >= PL::PREFETCH_MIN_BYTES) {
       // the tile of the CTA that starts one full wave later, into L2
@@ -707,7 +724,7 @@ fft_fwd_kernel(const double2* __restrict__ in, double2* __restrict__ out, long l
     const double2* src = in + tile0 * N;
     for (int idx = tid; idx < tile_elems; idx += F::THREADS) {
       const int jj = idx / N, e = idx - jj * N;
-      const double2 v = __ldg(src + idx);
+      const double2 v = load_point(src + idx);
       sm[F::slot(jj, e)] = make_longlong2(__double_as_longlong(v.x), __double_as_longlong(v.y));
     }
     __syncthreads();
@@ -722,11 +739,11 @@ fft_fwd_kernel(const double2* __restrict__ in, double2* __restrict__ out, long l
       // predicated loads (2 instructions a point)
       const double2* src = in + (TPB == 1 || active ? tr : batch - 1) * N + t;
 #pragma unroll
-      for (int i = 0; i < P; ++i) raw[i] = __ldg(src + T * i);
+      for (int i = 0; i < P; ++i) raw[i] = load_point(src + T * i);
     } else {
       const double2* src = in + tr * N + t;
 #pragma unroll
-      for (int i = 0; i < P; ++i) raw[i] = active ? __ldg(src + T * i) : make_double2(0.0, 0.0);
+      for (int i = 0; i < P; ++i) raw[i] = active ? load_point(src + T * i) : make_double2(0.0, 0.0);
     }
   }
 
