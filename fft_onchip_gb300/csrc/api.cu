@@ -307,7 +307,7 @@ fftoc_status launch_fwd(int n, const double* in, double* out, int64_t batch, int
   long long bl = (long long)batch;
   int* err = ds->err;
   void* args[] = {(void*)&in2, (void*)&out2, (void*)&bl, (void*)&tw, (void*)&err};
-  cudaError_t e = launch_overlapped(d.fn, (unsigned)blocks, d.threads, d.smem, args, stream);
+  cudaError_t e = launch_overlapped(d.fn, (unsigned)blocks, cap, d.threads, d.smem, args, stream);
   if (e != cudaSuccess) return cuda_fail(e, "cudaLaunchKernel");
   return FFTOC_OK;
 }

@@ -301,8 +301,10 @@ __device__ __forceinline__ int fx_transform_max(int em, int tid, int j, int* red
 // Programmatic dependent launch (launch_plan): a kernel may start while the one
 // before it in its stream drains.  after_previous() waits for that kernel's
 // completion and must come before any access to the caller's buffers;
-// allow_next() lets the next kernel's CTAs take the places that this grid no
-// longer needs (they wait at their own after_previous()).
+// allow_next(), after it, lets the next kernel's CTAs take the places that this
+// grid does not need (they wait at their own after_previous(); called before
+// the wait, it would let a chain of small grids pile up on the device, on
+// whichever SMs have room: 9.2 instead of 5.4 us for 1/3 of a wave of N = 512).
 __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // A point of the caller's input.  Not __ldg: the compiler takes read-only loads
@@ -688,8 +690,8 @@ fft_fwd_kernel(const double2* __restrict__ in, double2* __restrict__ out, long l
   extern __shared__ __align__(16) unsigned char smem_raw[];
   longlong2* sm = reinterpret_cast<longlong2*>(smem_raw);
 
-  allow_next();
   after_previous();
+  allow_next();
   if constexpr (PL::PREFETCH) {
     if (threadIdx.x == 0 && batch * (PL::N * 16) >= PL::PREFETCH_MIN_BYTES) {
       // the tile of the CTA that starts one full wave later, into L2

@@ -105,8 +105,8 @@ fft_fwd_persistent(const double2* __restrict__ in, double2* __restrict__ out, lo
     bulk_load(smem_raw + s * C::STAGE_BYTES, in + t0 * N, bytes, &bars[s]);
   };
 
-  allow_next();
   after_previous();
+  allow_next();
   // prologue: the first NSTAGE-1 tiles of this CTA
   if (tid == 0) {
     for (int s = 0; s < NSTAGE - 1; ++s) {

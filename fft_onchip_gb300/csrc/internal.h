@@ -127,10 +127,16 @@ inline cudaError_t fit_carveout(const void* fn, int threads, int smem, int* bloc
 // caller's buffers: it may be scheduled while the kernel before it in the
 // stream drains, which hides the launch and the fill of the first wave: 2-4 us
 // a call back to back (N = 64, 64 MiB: 28.6 -> 26.0 us; N = 1024, 82 MB: 41.0
-// -> 38.4 us).  The split-form kernels are launched without it: their CTAs
+// -> 38.4 us; 1,024 transforms of 512 points: 8.2 -> 5.4 us).
+// `wave` is the number of CTAs that fit the device at once.  A grid of 1/2 to
+// 2/3 of it is launched without the overlap: two such grids do not fit
+// together, so the next one's CTAs crowd on some SMs, and back to back that
+// measured up to 14 % slower at N = 256, 512, 1024 and 2048 (7-15 % faster at
+// 64, 128 and 4096); below and above the overlap wins at every N, by 3-70 %.
+// The split-form kernels are launched without it: their CTAs
 // stay for the whole grid, and they measured 1-2 % slower with it.
-inline cudaError_t launch_overlapped(const void* fn, unsigned blocks, int threads, int smem, void** args,
-                                     cudaStream_t stream) {
+inline cudaError_t launch_overlapped(const void* fn, unsigned blocks, long long wave, int threads, int smem,
+                                     void** args, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3((unsigned)threads);
@@ -140,7 +146,7 @@ inline cudaError_t launch_overlapped(const void* fn, unsigned blocks, int thread
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2LL * blocks > wave && 25LL * blocks <= 17 * wave ? 0 : 1;
   return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
