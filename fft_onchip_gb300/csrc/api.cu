@@ -7,6 +7,7 @@
 // (threads, UPB), and aborts the process through gpuErrchk
 // (includes/common.cuh:3-13) on any CUDA error.  This library instead returns
 // a status, keeps a per-thread message, and sizes the grid from the batch.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -177,7 +178,7 @@ void init_device(DeviceState& ds) {
     for (int i = 0; i < kNumSizes; ++i)
       for (int v = 0; v < ds.var[eng][i].count; ++v) {
         KernelDesc& d = ds.var[eng][i].v[v];
-        cudaError_t e = cudaFuncSetAttribute(d.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem);
+        cudaError_t e = allow_shared(d.fn, d.smem);
         // persistent grids are sized from the resident CTAs per SM
         if (e == cudaSuccess && d.persistent) e = fit_carveout(d.fn, d.threads, d.smem, &d.blocks_per_sm);
         else if (e == cudaSuccess)
@@ -270,8 +271,9 @@ fftoc_status device_plan_resources(int slot, int idx, int var, const void** tw, 
   return FFTOC_OK;
 }
 
+// `host`: in and out are device addresses of pinned host memory (launch_fwd_host).
 fftoc_status launch_fwd(int n, const double* in, double* out, int64_t batch, int engine, cudaStream_t stream,
-                        int variant = -1) {
+                        int variant = -1, bool host = false) {
   const int idx = size_index(n);
   if (idx < 0) return fail(FFTOC_ERR_INVALID_SIZE, "n=" + std::to_string(n) + " is not one of 8,16,...,4096");
   if (batch < 0) return fail(FFTOC_ERR_INVALID_VALUE, "batch must be >= 0");
@@ -299,19 +301,53 @@ fftoc_status launch_fwd(int n, const double* in, double* out, int64_t batch, int
   const KernelDesc& d = ds->var[slot][idx].v[var];
   const void* tw = ds->tw[slot][idx][var];
   const long long tiles = (batch + d.tpb - 1) / d.tpb;
-  const long long cap = (long long)ds->sms * d.blocks_per_sm;
+  const int smem = host && d.smem < kDirectSmem ? kDirectSmem : d.smem;
+  const long long cap = (long long)ds->sms * (smem > d.smem ? 1 : d.blocks_per_sm);
   const long long blocks = d.persistent ? (tiles < cap ? tiles : cap) : tiles;
   if (blocks > 0x7FFFFFFFLL) return fail(FFTOC_ERR_INVALID_VALUE, "batch too large for one launch");
   const double2* in2 = reinterpret_cast<const double2*>(in);
   double2* out2 = reinterpret_cast<double2*>(out);
   long long bl = (long long)batch;
   int* err = ds->err;
-  void* args[] = {(void*)&in2, (void*)&out2, (void*)&bl, (void*)&tw, (void*)&err};
-  cudaError_t e = launch_overlapped(d.fn, (unsigned)blocks, cap, d.threads, d.smem, args, stream);
+  int prefetch = host ? 0 : 1;
+  void* args[] = {(void*)&in2, (void*)&out2, (void*)&bl, (void*)&tw, (void*)&err, (void*)&prefetch};
+  cudaError_t e = launch_overlapped(d.fn, (unsigned)blocks, cap, d.threads, smem, args, stream);
   if (e != cudaSuccess) return cuda_fail(e, "cudaLaunchKernel");
   return FFTOC_OK;
 }
 
+// Largest batch that plans which spread a warp's access over many transforms
+// (N = 16 and 32, 64- and 128-byte pieces) take straight from host memory: over
+// the link the pieces cost more than the copies' own overheads at 1 GB (7.0 and
+// 7.6 ms against 6.5 staged), less up to some 200 MB (82 MB: 593 and 666 us
+// against 810).
+constexpr uintptr_t kDirectIoHostBytes = (uintptr_t)128 << 20;
+
+// The device address of `bytes` of host memory at p if all of it is pinned and
+// mapped (its first and last points are, at one distance from their addresses),
+// else null.
+void* mapped_host(const void* p, size_t bytes) {
+  cudaPointerAttributes a, b;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess ||
+      cudaPointerGetAttributes(&b, static_cast<const char*>(p) + bytes - 16) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer || !b.devicePointer) return nullptr;
+  return static_cast<char*>(b.devicePointer) - static_cast<char*>(a.devicePointer) == (ptrdiff_t)(bytes - 16)
+             ? a.devicePointer
+             : nullptr;
+}
+
+// Host buffers.  The binary64 and fixed-point engines transform pinned memory
+// in place of it: one launch whose CTAs load their tile over the host link and
+// store the result over it.  One CTA per SM (kDirectSmem) keeps 2-10 MB in
+// flight, enough for the link's latency; with full occupancy the first wave
+// only reads and the last only writes, 20-80 MB each.  Measured on one GB300
+// against staging (which pays the copies' launches, and a chunk each way
+// outside the overlap), n = 256: 10 KB 15 us against 33, 4 MB 47 against 71, 82 MB 513 against 812, 1 GB
+// 6.0 ms against 6.5 (164-171 GB/s each way, the link's rate in both directions
+// at once).  Pageable memory and the other engines are staged.
 fftoc_status launch_fwd_host(int n, const double* h_in, double* h_out, int64_t batch, int engine,
                              cudaStream_t stream) {
   const int idx = size_index(n);
@@ -328,12 +364,26 @@ fftoc_status launch_fwd_host(int n, const double* h_in, double* h_out, int64_t b
   DeviceState* ds = nullptr;
   fftoc_status st = device_state(&ds);
   if (st != FFTOC_OK) return st;
+  void *d_in = mapped_host(h_in, bytes), *d_out = d_in;
+  if (d_in && h_out != h_in) d_out = mapped_host(h_out, bytes);
+  const int eng = resolve_engine(n, engine);
+  const int slot = eng == FFTOC_ENGINE_FX ? 1 : 0;
+  const KernelDesc& plan = ds->var[slot][idx].v[chosen_variant(slot, idx)];
+  if (d_in && d_out && (eng == FFTOC_ENGINE_FX || eng == FFTOC_ENGINE_F64) &&
+      !plan.persistent &&  // bulk copies stay on device memory
+      (!(plan.code_flags & FFTOC_CODE_DIRECT_IO) || bytes <= kDirectIoHostBytes))
+    return launch_fwd(n, static_cast<const double*>(d_in), static_cast<double*>(d_out), batch, engine, stream, -1, true);
   Staging& sg = ds->staging;
   std::call_once(sg.once, [&] { init_staging(sg); });
   if (sg.status != FFTOC_OK) return fail(sg.status, sg.error);
 
   std::lock_guard<std::mutex> lock(sg.mu);
-  const int64_t chunk = (int64_t)(Staging::kChunkBytes / ((size_t)n * 16));
+  // pinned memory: chunks of 1/6 of the batch (2 to 64 MiB) overlap both
+  // directions for most of the call (82 MB: 812 us with 64 MiB chunks, 620-640
+  // with 8-16 MiB); pageable copies do not overlap
+  size_t chunk_bytes = Staging::kChunkBytes;
+  if (d_in && d_out) chunk_bytes = std::min(chunk_bytes, std::max((size_t)bytes / 6, (size_t)2 << 20));
+  const int64_t chunk = (int64_t)(chunk_bytes / ((size_t)n * 16));
   cudaError_t e;
   if ((e = cudaEventRecord(sg.ev_start, stream)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
   if ((e = cudaStreamWaitEvent(sg.s_h2d, sg.ev_start, 0)) != cudaSuccess) return cuda_fail(e, "cudaStreamWaitEvent");

@@ -79,7 +79,7 @@ void setup(NoAllocDevice& nd, int dev) {
       nd.var[slot][i] = compiled_variants(slot)[i];
       for (int v = 0; v < nd.var[slot][i].count; ++v) {
         KernelDesc& d = nd.var[slot][i].v[v];
-        if ((e = cudaFuncSetAttribute(d.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem)) != cudaSuccess)
+        if ((e = allow_shared(d.fn, d.smem)) != cudaSuccess)
           return bad(e, "cudaFuncSetAttribute");
         if ((e = d.persistent ? fit_carveout(d.fn, d.threads, d.smem, &d.blocks_per_sm)
                               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.blocks_per_sm, d.fn, d.threads,
@@ -176,7 +176,8 @@ fftoc_status launch_fwd_host_noalloc(int n, const double* h_in, double* h_out, i
   double2* y = reinterpret_cast<double2*>(nd.scratch);
   long long bl = (long long)batch;
   int* err = nd.err;
-  void* args[] = {(void*)&x, (void*)&y, (void*)&bl, (void*)&tw, (void*)&err};
+  int prefetch = 1;
+  void* args[] = {(void*)&x, (void*)&y, (void*)&bl, (void*)&tw, (void*)&err, (void*)&prefetch};
   if ((e = cudaLaunchKernel(d.fn, dim3((unsigned)blocks), dim3(d.threads), args, (size_t)d.smem, stream)) != cudaSuccess)
     return set_error(FFTOC_ERR_CUDA, std::string("cudaLaunchKernel: ") + cudaGetErrorString(e));
   if ((e = cudaMemcpyAsync(h_out, nd.scratch, bytes, cudaMemcpyDeviceToHost, stream)) != cudaSuccess)

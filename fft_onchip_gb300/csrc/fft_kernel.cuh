@@ -680,7 +680,7 @@ __device__ __forceinline__ void fft_tile(const Tile& tl, const typename E::TW* _
 template <class E, class PL>
 __global__ void __launch_bounds__(Fft<E, PL>::THREADS, PL::MINB)
 fft_fwd_kernel(const double2* __restrict__ in, double2* __restrict__ out, long long batch,
-               const typename E::TW* __restrict__ tw, int* __restrict__ err) {
+               const typename E::TW* __restrict__ tw, int* __restrict__ err, int prefetch) {
   (void)err;  // no waits in this kernel; the argument keeps one launch signature
   using EK = PlanEngine<E, PL>;
   using F = Fft<EK, PL>;
@@ -693,7 +693,7 @@ fft_fwd_kernel(const double2* __restrict__ in, double2* __restrict__ out, long l
   after_previous();
   allow_next();
   if constexpr (PL::PREFETCH) {
-    if (threadIdx.x == 0 && batch * (PL::N * 16) >= PL::PREFETCH_MIN_BYTES) {
+    if (threadIdx.x == 0 && prefetch && batch * (PL::N * 16) >= PL::PREFETCH_MIN_BYTES) {
       // the tile of the CTA that starts one full wave later, into L2
       unsigned nsm;
       asm("mov.u32 %0, %%nsmid;" : "=r"(nsm));

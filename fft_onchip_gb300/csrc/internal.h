@@ -123,6 +123,16 @@ inline cudaError_t fit_carveout(const void* fn, int threads, int smem, int* bloc
   return cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
 }
 
+// Dynamic shared memory of a launch on host buffers: more than half of an
+// SM's, so that one CTA runs per SM (launch_fwd_host).
+constexpr int kDirectSmem = 115 << 10;
+// Dynamic shared-memory limit of a batched kernel: its own and that of its
+// launches on host buffers.  Every set-up of such a kernel sets this same
+// limit (the attribute belongs to the function, the last call wins).
+inline cudaError_t allow_shared(const void* fn, int smem) {
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem > kDirectSmem ? smem : kDirectSmem);
+}
+
 // Launch of a kernel that calls after_previous() before it touches the
 // caller's buffers: it may be scheduled while the kernel before it in the
 // stream drains, which hides the launch and the fill of the first wave: 2-4 us

@@ -124,16 +124,18 @@ fftoc_status fftoc_c2c_fwd_split(int n, const double *in, double *out, int64_t b
 
 /* Host buffers in and out (the reference harness's path: cudaMemcpy H2D,
  * launch, cudaMemcpy D2H — includes/testing.cuh:109-113,166-171).
- * h_in/h_out are HOST pointers (pinned memory gives overlapped, full-speed
- * copies; pageable memory works but copies synchronously), 16-byte aligned,
- * batch*n complex values each; h_in == h_out is allowed.  The batch is
- * streamed through the device in chunks of 64 MiB (H2D, transform and D2H
- * of consecutive chunks overlap on three internal streams).  The call is
- * ordered after earlier work on `stream` and `stream` is ordered after its
- * last copy: synchronise `stream` before reading h_out.  The first call on a
- * device allocates 192 MiB of device staging memory and the streams (make it
- * before any stream capture); calls from several host threads serialise
- * their enqueueing. */
+ * h_in/h_out are HOST pointers (pinned memory runs at the host link's rate;
+ * pageable memory works but copies synchronously), 16-byte aligned, batch*n
+ * complex values each; h_in == h_out is allowed.  With the binary64 and
+ * fixed-point engines, pinned buffers are transformed by one kernel on
+ * `stream` that loads and stores them over the host link.  Otherwise the batch
+ * is streamed through the device in chunks of at most 64 MiB (H2D, transform
+ * and D2H of consecutive chunks overlap on three internal streams): the first
+ * such call on a device allocates 192 MiB of device staging memory and the
+ * streams (make it before any stream capture), and calls from several host
+ * threads serialise their enqueueing.  Either way the call is ordered after
+ * earlier work on `stream` and `stream` is ordered after its last store:
+ * synchronise `stream` before reading h_out. */
 fftoc_status fftoc_c2c_fwd_host(int n, const double *h_in, double *h_out, int64_t batch, int engine,
                                 fftoc_stream stream);
 
