@@ -16,6 +16,13 @@
 // i + j <= 1 (TF32x2).  Twiddles (FP32 table from long-double values) and
 // the short last pass of radix 2/4/8 run on the CUDA cores in FP32.
 //
+// Bound by latency at 16 warps per SM (127 registers of points, operands and
+// accumulators; 45 % of the issue slots), so fewer instructions and loads issued
+// early both count.  1 GiB, before and after the six-instruction conversions,
+// the binary32 exponent scan and the loads ahead: BF16x3 N = 256 426 -> 338 us,
+// 512 447 -> 362, 2048 504 -> 390, 4096 640 -> 531 (6.4, 5.9, 5.5, 4.0 TB/s);
+// TF32x2 N = 4096 715 -> 611.
+//
 // CTA: 128*G threads = G groups of 128 butterflies (one thread per butterfly
 // row); thread 0 issues the G*12 MMAs of a pass and commits them to an
 // mbarrier that every thread waits on (bounded); each warp reads its 32 TMEM
@@ -81,8 +88,12 @@ struct SplitPlan {
   static constexpr int DATA_OFF = A_BYTES + B_BYTES;
   static constexpr int DATA_BYTES = TPB * NP * 8;
   static constexpr int RED_OFF = DATA_OFF + DATA_BYTES;  // per-transform exponent scratch
-  static constexpr int BAR_OFF = RED_OFF + ((TPB * 4 + 15) / 16) * 16;
+  static constexpr int BAR_OFF = RED_OFF + ((TPB * (T > 32 ? T / 32 : 1) * 4 + 15) / 16) * 16;
   static constexpr int SMEM = BAR_OFF + 8 * G + 8;  // one mbarrier per group + TMEM address slot
+  // Multi-pass plans load the next tile's points into registers during the last
+  // pass (measured 1-9 % faster from N = 32 up; 1 % slower for the one pass of
+  // N = 16, whose loads are the bottleneck).
+  static constexpr bool LOAD_AHEAD = NS > 1;
   // a transform's threads lie inside one 128-row group: the groups need no
   // CTA-wide barrier inside a tile
   static constexpr bool GROUP_LOCAL = T <= 128;
@@ -226,6 +237,25 @@ __device__ __forceinline__ float f64_to_f32_int(double v) {
   return __uint_as_float(bits | (hi & 0x80000000u));
 }
 
+// The same for a finite |v| < 2^64, in 6 instructions against 14: the sign-
+// cleared 64-bit word plus half a unit of the FP32 significand, rebiased; an
+// exponent below the FP32 range leaves at most 7 units of the smallest
+// subnormal (0 stays 0).
+__device__ __forceinline__ float f64_to_f32_near(double v) {
+  const unsigned hw = (unsigned)__double2hiint(v);
+  unsigned lo, hi;
+  asm("add.cc.u32 %0, %2, 0x10000000;\n\taddc.u32 %1, %3, 0xC8000000;"  // - (896 << 20)
+      : "=r"(lo), "=r"(hi)
+      : "r"((unsigned)__double2loint(v)), "r"(hw & 0x7FFFFFFFu));
+  return __uint_as_float(__funnelshift_l(lo, (unsigned)max((int)hi, 0), 3) | (hw & 0x80000000u));
+}
+
+// FP32 -> binary64 of a normal value (exact).
+__device__ __forceinline__ double f32_to_f64_normal(float f) {
+  const unsigned u = __float_as_uint(f);
+  return __hiloint2double((int)((((u & 0x7FFFFFFFu) >> 3) + 0x38000000u) | (u & 0x80000000u)), (int)(u << 29));
+}
+
 // FP32 -> binary64 (exact) on the integer pipes; FP32 subnormals -> 0.
 __device__ __forceinline__ double f32_to_f64_int(float f) {
   const unsigned u = __float_as_uint(f);
@@ -283,6 +313,13 @@ __device__ __noinline__ void split_unscale_outputs(double2* dst, int t, int unsh
     }
 }
 
+// A point again, scaled by 2^shift (exact, binary64) before the general
+// conversion: transforms out of the FP32 range or not finite.  Out of line.
+__device__ __noinline__ float2 split_reload(const double2* p, int shift) {
+  const double2 v = *p;
+  return make_float2(f64_to_f32_int(ldexp(v.x, shift)), f64_to_f32_int(ldexp(v.y, shift)));
+}
+
 // Per-CTA state shared by the passes.
 struct SplitCtx {
   unsigned char* sA;
@@ -293,7 +330,15 @@ struct SplitCtx {
   unsigned tmem, idesc, phase;
   int tid, g, row, lane_block, j, t;
   bool failed;  // a bounded wait gave up (the tile loop ends after the tile)
+  const double2* nsrc;  // this thread's first point of the next tile
 };
+
+// A thread's 16 points of a tile.
+template <int T>
+__device__ __forceinline__ void split_load(double2 (&raw)[16], const double2* src) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i) raw[i] = __ldg(src + T * i);
+}
 
 // Barrier over the threads that share data inside a tile: the thread's
 // 128-row group when transforms do not span groups, else the CTA.
@@ -314,7 +359,7 @@ __device__ __forceinline__ void tile_sync(int g) {
 // end of the tile.
 template <int KIND, class PL, int G, int s>
 __device__ __forceinline__ void split_pass(SplitCtx& c, float (&re)[16], float (&im)[16], double2* dst, bool active,
-                                           int unshift, bool scaled) {
+                                           int unshift, bool scaled, bool special, double2 (&raw)[16]) {
   using SP = SplitPlan<KIND, PL, G>;
   using K = SplitT<KIND>;
   using L = OpLayout<K::ESIZE>;
@@ -365,6 +410,8 @@ __device__ __forceinline__ void split_pass(SplitCtx& c, float (&re)[16], float (
                        smem_u32(c.bar + c.g))
                    : "memory");
     }
+    // the next tile's points, while the MMAs run and the thread's own are gone
+    if constexpr (s == NS - 1 && SP::LOAD_AHEAD) split_load<T>(raw, c.nsrc);
     if (!c.failed && !mbar_wait_bounded(c.bar + c.g, c.phase, kWaitLimitNs)) c.failed = true;
     c.phase ^= 1;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -377,6 +424,7 @@ __device__ __forceinline__ void split_pass(SplitCtx& c, float (&re)[16], float (
     }
   } else {
     // last pass of radix 2/4/8 on the CUDA cores: 16/R butterflies per thread
+    split_load<T>(raw, c.nsrc);
 #pragma unroll
     for (int b = 0; b < Bq; ++b) {
       const int tp = c.t + T * b;
@@ -404,18 +452,35 @@ __device__ __forceinline__ void split_pass(SplitCtx& c, float (&re)[16], float (
       }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");  // this pass's TMEM reads precede the next MMAs
     tile_sync<SP::GROUP_LOCAL>(c.g);
-    split_pass<KIND, PL, G, s + 1>(c, re, im, dst, active, unshift, scaled);
+    split_pass<KIND, PL, G, s + 1>(c, re, im, dst, active, unshift, scaled, special, raw);
   } else {
     if (active) {
+      // zeros (and subnormals) and non-finite transforms take the general
+      // conversion: one minimum over the thread's values decides
+      float low = __uint_as_float(0x7F800000u);
 #pragma unroll
-      for (int b = 0; b < Bq; ++b)
+      for (int i = 0; i < 16; ++i) asm("min.f32 %0, %0, %1, %2;" : "+f"(low) : "f"(fabsf(re[i])), "f"(fabsf(im[i])));
+      if (!special && low >= 0x1p-126f) {
 #pragma unroll
-        for (int m = 0; m < R; ++m) {
+        for (int b = 0; b < Bq; ++b) {
           const int tp = c.t + T * b;
           const int k = tp & (p - 1);
-          const double xr = f32_to_f64_int(re[b + Bq * m]), xi = f32_to_f64_int(im[b + Bq * m]);
-          dst[(tp - k) * R + k + m * p] = make_double2(xr, xi);
+          double2* q = dst + (tp - k) * R + k;
+#pragma unroll
+          for (int m = 0; m < R; ++m)
+            q[m * p] = make_double2(f32_to_f64_normal(re[b + Bq * m]), f32_to_f64_normal(im[b + Bq * m]));
         }
+      } else {
+#pragma unroll
+        for (int b = 0; b < Bq; ++b) {
+          const int tp = c.t + T * b;
+          const int k = tp & (p - 1);
+          double2* q = dst + (tp - k) * R + k;
+#pragma unroll
+          for (int m = 0; m < R; ++m)
+            q[m * p] = make_double2(f32_to_f64_int(re[b + Bq * m]), f32_to_f64_int(im[b + Bq * m]));
+        }
+      }
       // rare transforms scaled at the input: undo the scale in place, out of
       // line (an if-converted ldexp would occupy the FP64 pipe for every value)
       if (scaled) split_unscale_outputs<T, R, Bq, p>(dst, c.t, unshift);
@@ -469,46 +534,45 @@ fft_split_kernel(const double2* __restrict__ in, double2* __restrict__ out, long
   c.failed = false;
 
   const long long ntiles = (batch + TPB - 1) / TPB;
+  double2 raw[16];  // the tile's points
+  if constexpr (SP::LOAD_AHEAD) {
+    const long long tr = (long long)blockIdx.x * TPB + c.j;
+    split_load<T>(raw, in + (tr < batch ? tr : batch - 1) * N + c.t);
+  }
   for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     if (c.tid == 0) prefetch_next_tile<N, TPB>(in, tile, batch);
     const long long tr = tile * TPB + c.j;
     const bool active = tr < batch;
-    // ---- load: point i of this thread is element t + T*i; per-transform
-    // power-of-two scale when the largest magnitude is outside [2^-60, 2^60]
-    double2 raw[16];
-    const double2* src = in + tr * N + c.t;
+    // ---- load and convert: point i of this thread is element t + T*i;
+    // per-transform power-of-two scale when the largest magnitude is outside
+    // [2^-60, 2^60]
+    const double2* src = in + (active ? tr : batch - 1) * N + c.t;
+    const long long ntr = tr + (long long)gridDim.x * TPB;
+    c.nsrc = in + (ntr < batch ? ntr : batch - 1) * N + c.t;
+    if constexpr (!SP::LOAD_AHEAD) split_load<T>(raw, src);
+    float re[16], im[16];
+    int em, emin;
+    fx_exponent_range<16>(raw, em, emin);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) raw[i] = active ? __ldg(src + T * i) : make_double2(0.0, 0.0);
-    int em = 0;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) em = max(em, max(expo_of(hi_word(raw[i].x)), expo_of(hi_word(raw[i].y))));
-    if constexpr (T > 1 && T <= 32) {
-#pragma unroll
-      for (int o = T / 2; o > 0; o >>= 1) em = max(em, __shfl_xor_sync(0xffffffffu, em, o, T));
-    } else if constexpr (T > 32) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) em = max(em, __shfl_xor_sync(0xffffffffu, em, o));
-      if (c.tid < TPB) red[c.tid] = 0;
-      __syncthreads();
-      if ((c.tid & 31) == 0) atomicMax(&red[c.j], em);
-      __syncthreads();
-      em = red[c.j];
+    for (int i = 0; i < 16; ++i) {
+      re[i] = f64_to_f32_near(raw[i].x);
+      im[i] = f64_to_f32_near(raw[i].y);
     }
+    em = fx_transform_max<T, TPB>(em, c.tid, c.j, red);
     // largest magnitude in [2^(em-1023), 2^(em-1022)); outside [2^-60, 2^60]
     // (or all subnormal, em = 0) scale it to ~1 by an exact power of two
     const bool scaled = em < 2047 && (em > 1023 + 60 || em < 1023 - 60);
     const int shift = scaled ? (em == 0 ? 1023 + 52 : 1023 - em) : 0;
-    if (scaled) {  // rare: exact binary64 scaling by 2^shift
+    const bool special = em == 2047;
+    if (scaled || special) {  // rare
 #pragma unroll
-      for (int i = 0; i < 16; ++i) raw[i] = make_double2(ldexp(raw[i].x, shift), ldexp(raw[i].y, shift));
+      for (int i = 0; i < 16; ++i) {
+        const float2 v = split_reload(src + T * i, shift);
+        re[i] = v.x;
+        im[i] = v.y;
+      }
     }
-    float re[16], im[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      re[i] = f64_to_f32_int(raw[i].x);
-      im[i] = f64_to_f32_int(raw[i].y);
-    }
-    split_pass<KIND, PL, G, 0>(c, re, im, out + tr * N, active, -shift, scaled);
+    split_pass<KIND, PL, G, 0>(c, re, im, out + tr * N, active, -shift, scaled, special, raw);
     // exchange buffer and exponent scratch free for the next tile; stop after
     // a bounded wait gave up anywhere in the CTA
     if (__syncthreads_or(c.failed)) {
