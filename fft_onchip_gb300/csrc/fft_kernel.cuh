@@ -39,6 +39,17 @@ template <int N> struct FxTrunc {
   static constexpr bool value = N <= 32;
 };
 
+// Sizes whose kernels convert threads with widely spread values by fx_in_far
+// instead of the general conversion (values over twelve decades leave the fast
+// path in most threads).  Same values, one more block of code: measured 5 %
+// faster on such data at N = 64, 128 and 1024 (1 GiB, log-uniform in [1e-6, 1e6]:
+// 365 -> 347, 385 -> 366, 517 -> 490 us) with ordinary data unchanged; at 256,
+// 512 and 2048 3-5 % faster there but up to 1 % slower on ordinary data, at 4096
+// no faster.
+template <int N> struct FxFar {
+  static constexpr bool value = N == 64 || N == 128 || N == 1024;
+};
+
 // --- binary64 <-> block fixed point -------------------------------------------
 FFTOC_HD unsigned hi_word(double v) {
 #ifdef __CUDA_ARCH__
@@ -168,6 +179,31 @@ FFTOC_HD long long fx_in_near(unsigned hw, unsigned lw, int eref) {
   return (long long)(((unsigned long long)hi << 32) | lo);
 }
 
+// Conversion of a normal value at any distance below the transform's largest
+// exponent, bit-identical to fx_in (floor): from 32 bits down the 96-bit word
+// is taken one word further up, and past 63 it is the sign.  5 instructions
+// more than fx_in_near, about 8 fewer than fx_in.
+FFTOC_HD long long fx_in_far(unsigned hw, unsigned lw, int eref) {
+  const unsigned S = (unsigned)((int)hw >> 31);
+  unsigned mh = (hw & 0xFFFFFu) ^ (S ^ 0x100000u);
+  unsigned l = lw ^ S;
+  const int d0 = eref - expo_of(hw), d = d0 < 63 ? d0 : 63;
+  if (d & 32) {
+    l = mh;
+    mh = S;
+  }
+#ifdef __CUDA_ARCH__
+  unsigned lo, hi;
+  asm("shf.r.wrap.b32 %0, %1, %2, %3;" : "=r"(lo) : "r"(l), "r"(mh), "r"(d));
+  asm("shf.r.wrap.b32 %0, %1, %2, %3;" : "=r"(hi) : "r"(mh), "r"(S), "r"(d));
+#else
+  const unsigned sh = (unsigned)d & 31u;
+  const unsigned lo = (unsigned)((((unsigned long long)mh << 32) | l) >> sh);
+  const unsigned hi = (unsigned)((((unsigned long long)S << 32) | mh) >> sh);
+#endif
+  return (long long)(((unsigned long long)hi << 32) | lo);
+}
+
 // The truncating fast conversion (bit-identical to fx_in<true> on the same
 // domain): the shifted magnitude, negated for a negative value.
 FFTOC_HD long long fx_in_near_trunc(unsigned hw, unsigned lw, int eref) {
@@ -236,11 +272,12 @@ FFTOC_HD void fx_exponent_range(const double2 (&raw)[P], int& emax, int& emin) {
 }
 
 // Convert a thread's P raw points; the fast path is taken when every value is
-// normal and within 2^31 of the transform maximum (the usual case).  emin is
-// the thread's smallest biased exponent (fx_exponent_range).
+// normal and within 2^31 of the transform maximum (the usual case), the next
+// (FAR, fx_in_far) when every value is normal.  emin is the thread's smallest
+// biased exponent (fx_exponent_range).
 // OUTLINE: the other path calls the out-of-line fx_in_slow.  TRUNC: the
 // size's rounding (FxTrunc).
-template <int P, bool OUTLINE = false, bool TRUNC = false>
+template <int P, bool OUTLINE = false, bool TRUNC = false, bool FAR = false>
 FFTOC_HD void fx_convert_in(const double2 (&raw)[P], long long (&re)[P], long long (&im)[P], int eref, int emin) {
   if (emin >= 1 && eref - emin < 32) {
 #pragma unroll
@@ -252,6 +289,12 @@ FFTOC_HD void fx_convert_in(const double2 (&raw)[P], long long (&re)[P], long lo
         re[i] = fx_in_near(hi_word(raw[i].x), lo_word(raw[i].x), eref);
         im[i] = fx_in_near(hi_word(raw[i].y), lo_word(raw[i].y), eref);
       }
+    }
+  } else if (FAR && emin >= 1) {
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      re[i] = fx_in_far(hi_word(raw[i].x), lo_word(raw[i].x), eref);
+      im[i] = fx_in_far(hi_word(raw[i].y), lo_word(raw[i].y), eref);
     }
   } else if constexpr (OUTLINE) {
 #pragma unroll
@@ -572,7 +615,7 @@ __device__ __forceinline__ void fft_tile(const Tile& tl, const typename E::TW* _
     K = sc.K;
     kshift = sc.kshift;
     slow = sc.slow;
-    fx_convert_in<P, false, TR>(raw, re, im, sc.eref, emin);
+    fx_convert_in<P, false, TR, FxFar<N>::value>(raw, re, im, sc.eref, emin);
   }
 
   if constexpr (F::STAGED) __syncthreads();  // staging buffer is reused by the passes
@@ -766,7 +809,7 @@ fft_fwd_kernel(const double2* __restrict__ in, double2* __restrict__ out, long l
     K = sc.K;
     kshift = sc.kshift;
     slow = sc.slow;
-    fx_convert_in<P, PL::OUTLINE_SLOW_IN, TR>(raw, re, im, sc.eref, emin);
+    fx_convert_in<P, PL::OUTLINE_SLOW_IN, TR, FxFar<N>::value>(raw, re, im, sc.eref, emin);
   }
 
   if constexpr (F::STAGED) __syncthreads();  // staging buffer is reused by the passes

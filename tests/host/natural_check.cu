@@ -226,8 +226,25 @@ static double check_plan(std::mt19937_64& g, const int* radix, int passes) {
   return worst;
 }
 
+// fx_in_far against fx_in over its domain: normal values from the transform's
+// largest exponent (zero distance) to far below it.  Returns the mismatches.
+static long long check_in_far(std::mt19937_64& g) {
+  long long bad = 0;
+  for (int t = 0; t < 1000000; ++t) {
+    const int em = 1 + (int)(g() % 2046), below = (int)(g() % (t & 1 ? 70 : 2046));
+    const int eref = em + (t % 3 == 0 ? 5 : 0);  // 53 and 48 input bits
+    const int e = em - below < 1 ? 1 : em - below;
+    const unsigned long long bits = g();
+    const unsigned hw = ((unsigned)(bits >> 32) & 0x800FFFFFu) | ((unsigned)e << 20);
+    const unsigned lw = t % 5 == 0 ? 0u : (unsigned)bits;
+    if (fx_in_far(hw, lw, eref) != fx_in<false>(hw, lw, eref)) ++bad;
+  }
+  return bad;
+}
+
 int main() {
   std::mt19937_64 g(20240607);
+  printf("in_far_mismatch %lld\n", check_in_far(g));
   printf("cmul_quarter_units %.4f\n", check_cmul<true>(g));
   printf("cmul_units %.4f\n", check_cmul<false>(g));
   printf("mulh_units %.4f\n", check_mulh(g));

@@ -46,6 +46,10 @@ def test_products_and_small_dfts(report, name, bound):
     assert report[name] < bound
 
 
+def test_far_input_conversion(report):
+    assert report["in_far_mismatch"] == 0
+
+
 def test_whole_plans_at_the_largest_scale(report):
     # at most 7 units a pass at the last pass's scale (2^-49 of the largest
     # input), three passes with twiddles, outputs of at least sqrt(N) times the
