@@ -138,14 +138,15 @@ void setup(SplitDevice& sd, int dev) {
       kd.passes = d.passes;
       for (int r = 0; r < 4; ++r) kd.radix[r] = d.radix[r];
       kd.tw_entries = d.tw_entries;
+      kd.natural = k == 2 ? 1 : 0;
       std::vector<double> f64;
       std::vector<int> fx;
       twiddle_tables(kd, f64, fx);
       const void* src;
       size_t bytes;
       std::vector<float> f32(f64.size() > 0 ? f64.size() : 2, 0.f);
-      if (k == 2) {  // exact slices: the fixed-point engine's 60-bit limb twiddles
-        if (fx.empty()) fx.assign(4, 0);
+      if (k == 2) {  // exact slices: the fixed-point engine's twiddles on the natural words
+        if (fx.empty()) fx.assign(6, 0);
         src = fx.data();
         bytes = fx.size() * 4;
       } else {

@@ -2,11 +2,12 @@
 // with products that are exact in FP32, for relative errors ~1e-14.
 //
 // Data stay in 64-bit block fixed point (per-transform power-of-two scale,
-// 60-bit limb twiddles on the CUDA cores).  A radix-16 pass's inputs are
-// below 2^BS: BS = B (the fixed-point engine's block bound) for the first
-// pass, 59 for later ones.  Each butterfly input x is cut to its top 49 bits,
-// t = x >> (BS - 48), and written as six balanced digits,
-// t = sum_i d_i 2^(8(5-i)), d_i in [-128, 127] for i >= 1 and d_0 in
+// twiddle products of the fixed-point engine on the CUDA cores).  A radix-16
+// pass's inputs are below 2^BS: BS = B (the fixed-point engine's block bound)
+// for the first pass, 57 for later ones, whose twiddle products are at quarter
+// scale (the cut drops more than those two bits).  Each butterfly input x is
+// cut to its top 49 bits, t = x >> (BS - 48), and written as six balanced
+// digits, t = sum_i d_i 2^(8(5-i)), d_i in [-128, 127] for i >= 1 and d_0 in
 // [-256, 256]: the offset-binary digits of u = t + 0x1008080808080 (bytes
 // 0..4 offset by 128, bits 40..49 by 256), each turned into the FP16 value
 // 1024 + digit by a byte permute and brought to its signed value by one FP16
@@ -23,9 +24,9 @@
 // kept as the next pass's input: each pass rescales the transform by a power
 // of two, accounted for in the output conversion.  Bounds by modulus: inputs
 // of modulus below sqrt2 2^BS give |C| <= 2^(54-BS) 16 sqrt2 2^BS = 2^58.5;
-// twiddles keep the modulus, so later passes cut at BS = 59 and give
-// |C| <= 2^-5 16 2^58.5 = 2^57.5, and a radix-2/4/8 last pass ends below
-// 2^61.5 (inside int64; its constant products see at most 2^59.5).
+// quarter-scale twiddle products take it to 2^56.5, so later passes cut at
+// BS = 57 and give |C| <= 2^-3 16 2^56.5 = 2^57.5, and a radix-2/4/8 last pass,
+// on full-scale products, ends below 2^61.5 (inside int64).
 //
 // Operand layout (FP16, K-major core matrices of 8 rows x 16 bytes).  The A
 // operand of a 128-row group is three K blocks, one per digit pair
@@ -42,6 +43,14 @@
 // Two threads serve each butterfly row: half h holds inputs and outputs
 // 8h..8h+7, writes their A digits and reads its 16 accumulator columns of
 // each order.
+//
+// Bound by latency and by the integer pipes (both 35 to 45 % busy, 16 warps per
+// SM, the limit of the registers and of the exchange buffers).  Products on
+// the natural 32-bit words at quarter scale instead of 30-bit limbs, one
+// binary32-ordered exponent range for the maximum and the fast-path test, and
+// the combination of the slices in two instructions less took 2^26 points from
+// 687, 641, 649, 791, 897, 936, 963 and 1380 us (N = 32 to 4096) to 627, 619,
+// 629, 755, 853, 883, 900 and 1348 us.
 #pragma once
 #include <cuda_fp16.h>
 
@@ -58,7 +67,7 @@ constexpr int kSplitExact = 3;
 constexpr int kExactDigits = 6;  // 8-bit digits per operand
 constexpr int kExactOrders = 6;  // slice orders s = 0..5 kept (21 digit pairs)
 constexpr int kExactBlocks = 3;  // digit pairs per operand row
-constexpr int kExactBound = 59;  // components of radix-16 pass outputs are below 2^59
+constexpr int kExactBound = 57;  // components of a later radix-16 pass's twiddled inputs are below 2^57
 
 template <class PL, int G>
 struct ExactPlan {
@@ -88,10 +97,10 @@ struct ExactPlan {
   static constexpr int TMEM_COLS = G == 1 ? 256 : 512;
   static_assert(G <= 2, "at most two 128-row groups");
   // radix-16 passes; the first scales the transform by 2^(54 - B), each
-  // later one by 2^(54 - 59), so outputs are y 2^(K + OUT_SHIFT) for the input
-  // scale 2^K
+  // later one by 2^-2 (its twiddle products) and 2^(54 - 57), so outputs are
+  // y 2^(K + OUT_SHIFT) for the input scale 2^K
   static constexpr int NR16 = PL::R[NS - 1] == 16 ? NS : NS - 1;
-  static constexpr int OUT_SHIFT = (B - 54) + (kExactBound - 54) * (NR16 - 1);
+  static constexpr int OUT_SHIFT = (B - 54) + (kExactBound + 2 - 54) * (NR16 - 1);
   __device__ __forceinline__ static int slot(int j, int e) { return j * NP + e + (e >> SH); }
 };
 
@@ -143,16 +152,18 @@ __device__ __forceinline__ void exact_digit_words(long long x, unsigned& w0, uns
 // One output from the bit patterns x[s] of its six order accumulators.  The
 // accumulators start at 1.5 * 2^23 (exact_tmem_fill) and gather exact
 // integers a[s], |a[s]| < 2^22, so each stays in [2^23, 2^24) and
-// x[s] = 0x4B400000 + a[s].  Returns C = sum_s a[s] 2^(8(5-s)): pairs of
-// orders are combined in 32 bits, (x[2i] - M) 2^8 + x[2i+1] = a[2i] 2^8 +
-// a[2i+1] + M, which lies in [0, 2^31) for i = 1, 2, the three pairs in 64
-// bits with one constant for the M terms.
+// x[s] = M + a[s], M = 0x4B400000.  Returns C = sum_s a[s] 2^(8(5-s)): pairs of
+// orders are combined in 32 bits, x[2i] 2^8 + x[2i+1] = a[2i] 2^8 + a[2i+1] +
+// 257 M (mod 2^32), where 257 M = 0x8B400000 (mod 2^32) and |a[2i] 2^8 +
+// a[2i+1]| < 2^30 + 2^22, so as an unsigned word it does not wrap; the three
+// pairs in 64 bits with one constant for the M terms.
 FFTOC_HD long long exact_combine(unsigned x0, unsigned x1, unsigned x2, unsigned x3, unsigned x4, unsigned x5) {
   constexpr unsigned M = 0x4B400000u;
-  constexpr unsigned long long KC = ((unsigned long long)(257u * M) << 32) + ((unsigned long long)M << 16) + M;
-  const unsigned pa = x0 * 256u + x1;        // a0 2^8 + a1 + 257 M (mod 2^32)
-  const unsigned pb = (x2 - M) * 256u + x3;  // a2 2^8 + a3 + M
-  const unsigned pc = (x4 - M) * 256u + x5;  // a4 2^8 + a5 + M
+  constexpr unsigned long long M2 = 257u * M;
+  constexpr unsigned long long KC = (M2 << 32) + (M2 << 16) + M2;
+  const unsigned pa = x0 * 256u + x1;
+  const unsigned pb = x2 * 256u + x3;
+  const unsigned pc = x4 * 256u + x5;
   return (long long)(((unsigned long long)pb << 16) + pc + ((unsigned long long)pa << 32) - KC);
 }
 
@@ -242,6 +253,7 @@ struct ExactCtx {
   longlong2* data;
   unsigned long long* bar;  // this group's MMA barrier
   const int4* tw;
+  const int2* tws;          // limbs of -(wr + wi), behind the entries of tw
   unsigned tmem;            // this group's accumulators, lane 0
   unsigned tmem_rd;         // this thread's lanes and columns
   unsigned phase;
@@ -266,22 +278,70 @@ __device__ __forceinline__ void exact_load_inputs(double2 (&raw)[8], const doubl
 template <class PL, int s>
 constexpr bool EARLY_TW = s > 0 && s == PL::S - 1 && PL::R[s] == 16;
 
+// The same for a radix-2/4 second pass (at most 8 entries): 10 % faster at
+// N = 32 and 64; 2 to 9 % slower with eight rows of twiddles (N = 128) or
+// after a third pass (N = 512 and 1024).
+template <class PL, int s>
+constexpr bool EARLY_SMALL_TW = s == 1 && s == PL::S - 1 && PL::R[s] <= 4;
+
+// A radix-16 pass before a radix-2 one (N = 512) forms -(wr + wi) from its
+// 16-byte entries instead of loading it: 850 against 912 us at 2^26 points,
+// where the loaded form spills; 0.5 to 1 % slower at N = 1024 to 4096.
+template <class PL, int s>
+constexpr bool SUM_TW = s + 2 == PL::S && PL::R[s + 1 < PL::S ? s + 1 : s] == 2;
+
+// Limbs of -(wr + wi) = -(2 wr + (wi - wr)); |wr + wi| <= sqrt2 2^62.
+__device__ __forceinline__ int2 exact_tw_sum(const int4 w) {
+  const long long r = ((long long)w.x << 32) + w.y, d = ((long long)w.z << 32) + w.w;
+  int2 c;
+  EngFxN::split(-(2 * r + d), c.x, c.y);
+  return c;
+}
+
 // The twiddles of radix-16 pass s (s >= 1) for this thread's inputs
 // m = 8h + i: entry (m - 1) p + k (none for m = 0).
 template <class PL, int s>
-__device__ __forceinline__ void exact_load_twiddles(const ExactCtx& c, int4 (&w)[8]) {
+__device__ __forceinline__ void exact_load_twiddles(const ExactCtx& c, int4 (&w)[8], int2 (&ws)[8]) {
   constexpr int p = PL::span(s);
   const int k = c.t & (p - 1);
-  const int4* base = c.tw + PL::tw_offset(s) + k + 8 * c.h * p;
+  const int e = PL::tw_offset(s) + k + 8 * c.h * p;
 #pragma unroll
-  for (int i = 1; i < 8; ++i) w[i] = __ldg(base + (i - 1) * p);
-  w[0] = c.h ? __ldg(base - p) : w[1];
+  for (int i = 1; i < 8; ++i) {
+    w[i] = __ldg(c.tw + e + (i - 1) * p);
+    ws[i] = __ldg(c.tws + e + (i - 1) * p);
+  }
+  w[0] = c.h ? __ldg(c.tw + e - p) : w[1];
+  ws[0] = c.h ? __ldg(c.tws + e - p) : ws[1];
+}
+
+// The twiddles of a radix-2/4 last pass: those of input m >= 1 of butterfly b at
+// b + Bh (m - 1).
+template <class PL, int s>
+__device__ __forceinline__ void exact_load_small_twiddles(const ExactCtx& c, int4 (&w)[8], int2 (&ws)[8]) {
+  constexpr int p = PL::span(s), R = PL::R[s], Bh = 8 / R;
+#pragma unroll
+  for (int b = 0; b < Bh; ++b) {
+    const int e = PL::tw_offset(s) + ((c.t + PL::T * (c.h * Bh + b)) & (p - 1));
+#pragma unroll
+    for (int m = 1; m < R; ++m) {
+      w[b + Bh * (m - 1)] = __ldg(c.tw + e + (m - 1) * p);
+      ws[b + Bh * (m - 1)] = __ldg(c.tws + e + (m - 1) * p);
+    }
+  }
+}
+
+// One twiddle product, its entry e loaded at the product.
+template <class PL, int s, bool QUARTER>
+__device__ __forceinline__ void exact_cmul_at(const ExactCtx& c, long long& re, long long& im, int e) {
+  const int4 w = __ldg(c.tw + e);
+  if constexpr (SUM_TW<PL, s>) EngFxN::cmul<QUARTER>(re, im, w, exact_tw_sum(w));
+  else EngFxN::cmul<QUARTER>(re, im, w, __ldg(c.tws + e));
 }
 
 template <int R, int Bq, int... bs>
 __device__ __forceinline__ void exact_small_dfts(long long (&re)[8], long long (&im)[8],
                                                  std::integer_sequence<int, bs...>) {
-  (dft<EngFx, R, bs, Bq, 8>(re, im), ...);
+  (dft<EngFxN, R, bs, Bq, 8>(re, im), ...);
 }
 
 // Pass s of the plan.  Radix-16 passes: the half's 8 inputs (already in re/im
@@ -294,15 +354,15 @@ __device__ __forceinline__ void exact_small_dfts(long long (&re)[8], long long (
 // overlaps the pass.
 template <class PL, int G, int s>
 __device__ __forceinline__ void exact_pass(ExactCtx& c, long long (&re)[8], long long (&im)[8], const ExactOut& o,
-                                           double2 (&raw)[8], const int4 (&w)[8]) {
+                                           double2 (&raw)[8], const int4 (&w)[8], const int2 (&ws)[8]) {
   using XP = ExactPlan<PL, G>;
   constexpr int T = PL::T, NS = PL::S;
   constexpr int R = PL::R[s];
   constexpr int p = PL::span(s);
   static_assert(R == 16 || s == NS - 1, "radix 2/4/8 only in the last pass");
   static_assert(R == 16 || s > 0, "radix-16 first pass");
-  // input components of pass s: below 2^B (s = 0) or 2^59 (C of the
-  // previous pass, modulus <= 2^58.5, kept by the twiddle products)
+  // input components of pass s: below 2^B (s = 0) or 2^57 (C of the previous
+  // pass, modulus <= 2^58.5, times the quarter-scale twiddles)
   constexpr int BS = s == 0 ? XP::B : kExactBound;
   static_assert(R <= 8 || R == 16, "radix 2/4/8 last pass: outputs below 2^61.5");
   if constexpr (R == 16) {
@@ -315,14 +375,19 @@ __device__ __forceinline__ void exact_pass(ExactCtx& c, long long (&re)[8], long
       }
       if constexpr (EARLY_TW<PL, s>) {
 #pragma unroll
-        for (int i = 1; i < 8; ++i) EngFx::cmul(re[i], im[i], w[i]);
-        if (c.h) EngFx::cmul(re[0], im[0], w[0]);
+        for (int i = 1; i < 8; ++i) EngFxN::cmul<true>(re[i], im[i], w[i], ws[i]);
       } else {
-        const int k = c.t & (p - 1);
-        const int4* base = c.tw + PL::tw_offset(s) + k + (8 * c.h - 1) * p;  // input m = 8h + i: (m - 1) p
+        const int e = PL::tw_offset(s) + (c.t & (p - 1)) + (8 * c.h - 1) * p;  // input m = 8h + i: (m - 1) p
 #pragma unroll
-        for (int i = 1; i < 8; ++i) EngFx::cmul(re[i], im[i], __ldg(base + i * p));
-        if (c.h) EngFx::cmul(re[0], im[0], __ldg(base));
+        for (int i = 1; i < 8; ++i) exact_cmul_at<PL, s, true>(c, re[i], im[i], e + i * p);
+      }
+      if (c.h == 0) {  // input 0: no twiddle
+        re[0] >>= 2;
+        im[0] >>= 2;
+      } else if constexpr (EARLY_TW<PL, s>) {
+        EngFxN::cmul<true>(re[0], im[0], w[0], ws[0]);
+      } else {
+        exact_cmul_at<PL, s, true>(c, re[0], im[0], PL::tw_offset(s) + (c.t & (p - 1)) + 7 * p);
       }
     }
     // A digits: values 8h..8h+7 (real) are chunks 2h, 2h+1 of each block,
@@ -405,9 +470,13 @@ __device__ __forceinline__ void exact_pass(ExactCtx& c, long long (&re)[8], long
 #pragma unroll
     for (int b = 0; b < Bh; ++b) {
       const int tp = c.t + T * (c.h * Bh + b);
-      const int4* base = c.tw + PL::tw_offset(s) + (tp & (p - 1));
+      const int e = PL::tw_offset(s) + (tp & (p - 1));
 #pragma unroll
-      for (int m = 1; m < R; ++m) EngFx::cmul(re[b + Bh * m], im[b + Bh * m], __ldg(base + (m - 1) * p));
+      for (int m = 1; m < R; ++m) {
+        const int i = b + Bh * (m - 1);
+        if constexpr (EARLY_SMALL_TW<PL, s>) EngFxN::cmul<false>(re[i + Bh], im[i + Bh], w[i], ws[i]);
+        else exact_cmul_at<PL, s, false>(c, re[i + Bh], im[i + Bh], e + (m - 1) * p);
+      }
     }
     exact_small_dfts<R, Bh>(re, im, std::make_integer_sequence<int, Bh>{});
     if (o.active) {
@@ -423,20 +492,39 @@ __device__ __forceinline__ void exact_pass(ExactCtx& c, long long (&re)[8], long
   }
   if constexpr (s + 1 < NS) {
     int4 wn[8];
-    if constexpr (EARLY_TW<PL, s + 1>) exact_load_twiddles<PL, s + 1>(c, wn);
+    int2 wsn[8];
+    if constexpr (EARLY_TW<PL, s + 1>) exact_load_twiddles<PL, s + 1>(c, wn, wsn);
+    if constexpr (EARLY_SMALL_TW<PL, s + 1>) exact_load_small_twiddles<PL, s + 1>(c, wn, wsn);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    exact_pass<PL, G, s + 1>(c, re, im, o, raw, wn);
+    exact_pass<PL, G, s + 1>(c, re, im, o, raw, wn, wsn);
   }
 }
 
-// Largest sign-cleared high word of a thread's inputs: the exponent field
-// of its largest value, or for subnormals the position of the leading bit.
-__device__ __forceinline__ unsigned exact_high_max(const double2 (&raw)[8]) {
-  unsigned a = 0u;
+// Largest sign-cleared high word of a thread's inputs (the exponent field of
+// its largest value, or for subnormals the position of the leading bit) and
+// the smallest exponent field.  Ordered as binary32 values as in
+// fx_exponent_range, which does not flush subnormal words to zero.
+__device__ __forceinline__ unsigned exact_high_range(const double2 (&raw)[8], int& emin) {
+  float fmax = 0.0f, fmin = __uint_as_float(0x7F800000u);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) a = max(a, max(hi_word(raw[i].x) & 0x7FFFFFFFu, hi_word(raw[i].y) & 0x7FFFFFFFu));
-  return a;
+  for (int i = 0; i < 8; ++i) {
+    const float a = fabsf(__uint_as_float(hi_word(raw[i].x))), b = fabsf(__uint_as_float(hi_word(raw[i].y)));
+    asm("max.NaN.f32 %0, %0, %1, %2;" : "+f"(fmax) : "f"(a), "f"(b));
+    asm("min.f32 %0, %0, %1, %2;" : "+f"(fmin) : "f"(a), "f"(b));
+  }
+  const unsigned a = __float_as_uint(fmax);
+  emin = (int)(__float_as_uint(fmin) >> 20);
+  if (a < 0x7F800000u) return a;
+  unsigned amax = 0u, amin = 0x7FFFFFFFu;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const unsigned x = hi_word(raw[i].x) & 0x7FFFFFFFu, y = hi_word(raw[i].y) & 0x7FFFFFFFu;
+    amax = max(amax, max(x, y));
+    amin = min(amin, min(x, y));
+  }
+  emin = (int)(amin >> 20);
+  return amax;
 }
 
 // Largest value of a over a transform's rows and both halves, in two steps
@@ -482,6 +570,7 @@ fft_exact_kernel(const double2* __restrict__ in, double2* __restrict__ out, long
   c.data = reinterpret_cast<longlong2*>(smem_exact + XP::DATA_OFF);
   c.bar = bars + g;
   c.tw = tw;
+  c.tws = reinterpret_cast<const int2*>(tw + PL::TW_COUNT);
   c.tid = tid;
   c.g = g;
   c.h = h;
@@ -499,11 +588,12 @@ fft_exact_kernel(const double2* __restrict__ in, double2* __restrict__ out, long
   }
   // the first tile's inputs and maximum (read after the set-up barrier)
   const long long ntiles = (batch + TPB - 1) / TPB;
+  int emin;        // smallest exponent field of raw
   double2 raw[8];  // the current tile's inputs, loaded during the previous tile
   {
     const long long tr = (long long)blockIdx.x * TPB + c.j;
     exact_load_inputs<T>(raw, in + (tr < batch ? tr : 0) * N + c.t + T * 8 * h, tr < batch);
-    exact_transform_put<T, TPB, XP::W>(exact_high_max(raw), h, c.j, c.t, red);
+    exact_transform_put<T, TPB, XP::W>(exact_high_range(raw, emin), h, c.j, c.t, red);
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
@@ -538,11 +628,11 @@ fft_exact_kernel(const double2* __restrict__ in, double2* __restrict__ out, long
       // its largest exponent field is then bitlen(at) + 44
 #pragma unroll
       for (int i = 0; i < 8; ++i) raw[i] = make_double2(raw[i].x * 0x1p64, raw[i].y * 0x1p64);
+      int unused;
+      fx_exponent_range<8>(raw, unused, emin);
       em = (32 - __clz(at)) + 44;
       kadj = -64;
     }
-    int em_thread, emin;
-    fx_exponent_range<8>(raw, em_thread, emin);
     const FxScale sc = fx_scale<XP::B>(em);
     long long re[8], im[8];
     fx_convert_in<8>(raw, re, im, sc.eref, emin);
@@ -551,9 +641,10 @@ fft_exact_kernel(const double2* __restrict__ in, double2* __restrict__ out, long
     const ExactOut o{out + tr * N, active, e_out < XP::B || e_out > 1983 + XP::B, sc.special,
                      (int)((unsigned)k_out << 20), k_out};
     const int4 w0[8] = {};
-    exact_pass<PL, G, 0>(c, re, im, o, raw, w0);
+    const int2 ws0[8] = {};
+    exact_pass<PL, G, 0>(c, re, im, o, raw, w0, ws0);
     // the next tile's maximum, read after the barrier
-    exact_transform_put<T, TPB, XP::W>(exact_high_max(raw), h, c.j, c.t, red);
+    exact_transform_put<T, TPB, XP::W>(exact_high_range(raw, emin), h, c.j, c.t, red);
     if (__syncthreads_or(c.failed)) {
       if (tid == 0) atomicOr(err, kErrTimeout);
       mbar_wait_bounded(c.bar, c.phase ^ 1, kWaitLimitNs);  // bounded drain of the MMAs in flight
