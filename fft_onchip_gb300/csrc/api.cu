@@ -126,7 +126,9 @@ void fxn_limbs(long double v, int* h, int* l) {
   *h = (int)((q - *l) >> 32);
 }
 
-// Twiddle table of a plan in each engine's layout.  f64: (cos, -sin) pairs.
+// Twiddle table of a plan in each engine's layout.  f64: (cos, -sin) pairs, or
+// (d.tangent) those of the upper half of a pass's inputs in EngF64's tangent
+// form.
 // fx, 4 ints per entry: 30-bit limbs of both parts, or (d.natural) the natural
 // limbs of wr and of wi - wr; there, behind all entries, 2 ints per entry: the
 // limbs of -(wr + wi).
@@ -143,6 +145,11 @@ void build_twiddles(const KernelDesc& d, std::vector<double>& f64, std::vector<i
         const int e = off + (m - 1) * p + k;
         f64[2 * e] = (double)c;
         f64[2 * e + 1] = (double)(-sn);
+        if (d.tangent && m >= R / 2) {
+          const bool turned = EngF64::tangent_turned(k * m, R * p);
+          f64[2 * e] = (double)(turned ? -sn : c);
+          f64[2 * e + 1] = (double)(turned ? c / sn : -sn / c);
+        }
         if (d.natural) {
           int* sum = &fx[4 * (size_t)d.tw_entries + 2 * e];
           fxn_limbs(c, &fx[4 * e], &fx[4 * e + 1]);

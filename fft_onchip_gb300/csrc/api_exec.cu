@@ -41,6 +41,7 @@ extern "C" fftoc_status fftoc_exec_twiddles(int n, int engine, const int radix[4
 
   KernelDesc d;
   d.natural = n >= kNaturalMinN ? 1 : 0;
+  d.tangent = eng == FFTOC_ENGINE_F64 ? 1 : 0;
   long long prod = 1;
   bool tail = false;  // an unused pass (1) was seen: only 1s may follow
   for (int s = 0; s < 4; ++s) {

@@ -400,6 +400,16 @@ struct Fft {
 #pragma unroll
         for (int m = 1; m < R; ++m)
           E::template cmul<QUARTER>(re[b + B * m], im[b + B * m], __ldg(base + (m - 1) * p), __ldg(sums + (m - 1) * p));
+      } else if constexpr (E::kId == EngF64::kId) {
+        constexpr int H = R / 2;
+#pragma unroll
+        for (int m = 1; m < H; ++m) E::cmul(re[b + B * m], im[b + B * m], __ldg(base + (m - 1) * p));
+#pragma unroll
+        for (int m = 0; m < H; ++m)
+          E::twiddled_sum(re[b + B * m], im[b + B * m], re[b + B * (m + H)], im[b + B * (m + H)],
+                          __ldg(base + (m + H - 1) * p), E::tangent_turned((m + H) * k, R * p));
+        f64_finish<R, b, B, P>(re, im);
+        return;
       } else {
 #pragma unroll
         for (int m = 1; m < R; ++m) {

@@ -30,6 +30,7 @@ struct KernelDesc {
   int radix[4] = {1, 1, 1, 1};
   int tw_entries = 0;        // twiddle table entries
   int natural = 0;           // 1: fixed-point table in the natural-word layout (EngFxN)
+  int tangent = 0;           // 1: binary64 table with EngF64's tangent forms
   int persistent = 0;        // 1: grid-stride persistent CTAs with TMA prefetch (extra error-flag argument)
   int stages = 0;            // shared-memory stages of the persistent kernel
   int blocks_per_sm = 0;     // resident CTAs per SM (filled at device set-up)

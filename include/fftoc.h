@@ -347,11 +347,11 @@ fftoc_status fftoc_onchip_run(int n, int engine, double *data, int64_t blocks, i
 /* Twiddle table for the device-side executors of <fftoc/exec.cuh> (the
  * FFTExec shape of includes/tensor_fft_64.cuh:12-45): the table of a plan of
  * size n whose passes have radices radix[0..3] (each 2, 4, 8 or 16, unused
- * passes 1 at the end), in the engine's layout (binary64 (cos, -sin), 16 bytes
- * per entry, or fixed-point limbs, 16 bytes for n <= 32 and 24 from 64 up: the
- * layout belongs to the <fftoc/exec.cuh> shipped with the library, so compile
- * executors against the header of the library they run with), in device memory of the current device
- * owned by the library until the process exits.  *table is NULL for a
+ * passes 1 at the end), in the engine's layout (binary64, 16 bytes per entry,
+ * or fixed-point limbs, 16 bytes for n <= 32 and 24 from 64 up: the layout
+ * belongs to the <fftoc/exec.cuh> shipped with the library, so compile
+ * executors against the header of the library they run with), in device memory
+ * of the current device owned by the library until the process exits.  *table is NULL for a
  * one-pass plan (no twiddles).  Engines: binary64, fixed point (AUTO
  * resolves to the latter).  Synchronous on first use of a plan. */
 fftoc_status fftoc_exec_twiddles(int n, int engine, const int radix[4], const void **table);
