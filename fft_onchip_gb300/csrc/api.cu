@@ -102,8 +102,8 @@ struct DeviceState {
   std::atomic<bool> ready{false};                 // set-up done and successful
 };
 
-// Plan chosen per (engine, size): process-wide, set by fftoc_plan_select or
-// fftoc_autotune; variant 0 until then.
+// Plan chosen per (engine, size), plus one: process-wide, set by
+// fftoc_plan_select or fftoc_autotune; 0 until then.
 std::atomic<int> g_choice[2][kNumSizes];
 
 const SizeVariants* host_variants(int eng_slot) {
@@ -264,7 +264,10 @@ int resolve_engine(int n, int engine) {
 // Accessors for other translation units (the allocation-free entry point).
 const SizeVariants* compiled_variants(int eng_slot) { return host_variants(eng_slot); }
 void twiddle_tables(const KernelDesc& d, std::vector<double>& f64, std::vector<int>& fx) { build_twiddles(d, f64, fx); }
-int chosen_variant(int eng_slot, int idx) { return g_choice[eng_slot][idx].load(std::memory_order_relaxed); }
+int chosen_variant(int eng_slot, int idx) {
+  const int c = g_choice[eng_slot][idx].load(std::memory_order_relaxed);
+  return c > 0 ? c - 1 : 0;
+}
 int resolved_engine(int n, int engine) { return resolve_engine(n, engine); }
 fftoc_status set_error(fftoc_status st, const std::string& msg) { return fail(st, msg); }
 fftoc_status device_plan_resources(int slot, int idx, int var, const void** tw, int** err, int* sms) {
@@ -276,6 +279,26 @@ fftoc_status device_plan_resources(int slot, int idx, int var, const void** tw, 
   *err = ds->err;
   *sms = ds->sms;
   return FFTOC_OK;
+}
+
+// Plan of a batch on device buffers: the chosen one for every batch, or while
+// none was chosen variant 0, and its SmallBatch<> plan up to that plan's limit.
+// The limits are where the two measured equal on 152 SMs, or where the larger
+// one's waves first beat it (back-to-back launches, us, variant 0 against the
+// small-batch plan, one transform and at the limit):
+//   N = 8     4.0 2.4    7.3 5.6 (77824)    256   6.2 3.5   63.6 58.8 (38912)
+//   16        2.9 2.2    3.5 3.4 (19456)    512   3.5 3.3    5.3 5.2 (760)
+//   32        4.5 2.3   15.7 15.3 (77824)   1024  4.2 3.8    6.3 6.2 (456)
+//   64        3.0 2.2    3.8 3.7 (4864)     2048  6.8 5.1   18.3 17.4 (912)
+//   128       5.6 3.5   60.2 55.8 (77824)
+// (4096: radix 8 in 512 threads 8.7 against 8.6, two barriers more: none.)
+int batch_variant(const DeviceState& ds, int slot, int idx, int64_t batch) {
+  if (g_choice[slot][idx].load(std::memory_order_relaxed) == 0) {
+    const SizeVariants& sv = ds.var[slot][idx];
+    for (int v = 0; v < sv.count; ++v)
+      if (sv.v[v].small_per_sm > 0) return batch <= (int64_t)sv.v[v].small_per_sm * ds.sms ? v : 0;
+  }
+  return chosen_variant(slot, idx);
 }
 
 // `host`: in and out are device addresses of pinned host memory (launch_fwd_host).
@@ -303,7 +326,7 @@ fftoc_status launch_fwd(int n, const double* in, double* out, int64_t batch, int
   fftoc_status st = device_state(&ds);
   if (st != FFTOC_OK) return st;
   const int slot = eng == FFTOC_ENGINE_FX ? 1 : 0;
-  const int var = variant >= 0 ? variant : g_choice[slot][idx].load(std::memory_order_relaxed);
+  const int var = variant >= 0 ? variant : batch_variant(*ds, slot, idx, batch);
   if (var >= ds->var[slot][idx].count) return fail(FFTOC_ERR_INVALID_VALUE, "no such plan variant");
   const KernelDesc& d = ds->var[slot][idx].v[var];
   const void* tw = ds->tw[slot][idx][var];
@@ -375,11 +398,15 @@ fftoc_status launch_fwd_host(int n, const double* h_in, double* h_out, int64_t b
   if (d_in && h_out != h_in) d_out = mapped_host(h_out, bytes);
   const int eng = resolve_engine(n, engine);
   const int slot = eng == FFTOC_ENGINE_FX ? 1 : 0;
-  const KernelDesc& plan = ds->var[slot][idx].v[chosen_variant(slot, idx)];
-  if (d_in && d_out && (eng == FFTOC_ENGINE_FX || eng == FFTOC_ENGINE_F64) &&
+  // one plan for the whole call, and not the small-batch one: the link bounds
+  // these, and the larger tiles keep more of it in flight
+  const bool planned = eng == FFTOC_ENGINE_FX || eng == FFTOC_ENGINE_F64;
+  const int var = planned ? chosen_variant(slot, idx) : -1;
+  const KernelDesc& plan = ds->var[slot][idx].v[planned ? var : 0];
+  if (d_in && d_out && planned &&
       !plan.persistent &&  // bulk copies stay on device memory
       (!(plan.code_flags & FFTOC_CODE_DIRECT_IO) || bytes <= kDirectIoHostBytes))
-    return launch_fwd(n, static_cast<const double*>(d_in), static_cast<double*>(d_out), batch, engine, stream, -1, true);
+    return launch_fwd(n, static_cast<const double*>(d_in), static_cast<double*>(d_out), batch, engine, stream, var, true);
   Staging& sg = ds->staging;
   std::call_once(sg.once, [&] { init_staging(sg); });
   if (sg.status != FFTOC_OK) return fail(sg.status, sg.error);
@@ -406,7 +433,8 @@ fftoc_status launch_fwd_host(int n, const double* h_in, double* h_out, int64_t b
       return cuda_fail(e, "cudaMemcpyAsync(H2D)");
     if ((e = cudaEventRecord(sg.ev_h2d[bi], sg.s_h2d)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
     if ((e = cudaStreamWaitEvent(sg.s_cmp, sg.ev_h2d[bi], 0)) != cudaSuccess) return cuda_fail(e, "cudaStreamWaitEvent");
-    st = launch_fwd(n, static_cast<const double*>(sg.buf[bi]), static_cast<double*>(sg.buf[bi]), cnt, engine, sg.s_cmp);
+    st = launch_fwd(n, static_cast<const double*>(sg.buf[bi]), static_cast<double*>(sg.buf[bi]), cnt, engine, sg.s_cmp,
+                    var);
     if (st != FFTOC_OK) return st;
     if ((e = cudaEventRecord(sg.ev_cmp[bi], sg.s_cmp)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
     if ((e = cudaStreamWaitEvent(sg.s_d2h, sg.ev_cmp[bi], 0)) != cudaSuccess) return cuda_fail(e, "cudaStreamWaitEvent");
@@ -437,7 +465,7 @@ fftoc_status plan_query(int n, int engine, int variant, fftoc_plan_info* info) {
   }
   const int slot = eng == FFTOC_ENGINE_FX ? 1 : 0;
   const SizeVariants& sv = host_variants(slot)[idx];
-  const int var = variant >= 0 ? variant : g_choice[slot][idx].load(std::memory_order_relaxed);
+  const int var = variant >= 0 ? variant : chosen_variant(slot, idx);
   if (var >= sv.count) return fail(FFTOC_ERR_INVALID_VALUE, "no such plan variant");
   const KernelDesc& d = sv.v[var];
   info->n = n;
@@ -496,7 +524,7 @@ fftoc_status plan_select(int n, int engine, int variant) {
   if (variant < 0) return fail(FFTOC_ERR_INVALID_VALUE, "variant must be >= 0");
   // engines with one plan per size (split forms, DMMA) have no choice to store
   if (info.engine == FFTOC_ENGINE_FX || info.engine == FFTOC_ENGINE_F64)
-    g_choice[info.engine == FFTOC_ENGINE_FX ? 1 : 0][size_index(n)].store(variant);
+    g_choice[info.engine == FFTOC_ENGINE_FX ? 1 : 0][size_index(n)].store(variant + 1);
   return FFTOC_OK;
 }
 
@@ -548,7 +576,7 @@ fftoc_status autotune(int n, int engine, int64_t batch, cudaStream_t stream, int
   if (st != FFTOC_OK) return st;
   if (e != cudaSuccess) return cuda_fail(e, "autotune");
   if (info.engine == FFTOC_ENGINE_FX || info.engine == FFTOC_ENGINE_F64)
-    g_choice[info.engine == FFTOC_ENGINE_FX ? 1 : 0][size_index(n)].store(bestv);
+    g_choice[info.engine == FFTOC_ENGINE_FX ? 1 : 0][size_index(n)].store(bestv + 1);
   if (best_variant) *best_variant = bestv;
   if (best_ms) *best_ms = best;
   return FFTOC_OK;

@@ -48,6 +48,7 @@ struct PlanT {
   static constexpr bool OUT_HI_ZERO = false;  // fixed point: zero test on the converted word (OutHiZero<>)
   static constexpr bool NO_STAGE = false;  // fewer than 8 threads per transform: direct HBM access (NoStage<>)
   static constexpr bool UNEVEN_DEFAULT = false;  // the uneven path's default plan for its size (UnevenDefault<>)
+  static constexpr int SMALL_PER_SM = 0;  // the size's plan for small batches (SmallBatch<>)
   static constexpr int R[4] = {R0, R1, R2, R3};
   static constexpr int S = (R0 > 1) + (R1 > 1) + (R2 > 1) + (R3 > 1);
   static constexpr int T = N / P;
@@ -371,6 +372,15 @@ struct NoStage : PL {
 template <class PL>
 struct UnevenDefault : PL {
   static constexpr bool UNEVEN_DEFAULT = true;
+};
+
+// The plan of batches of up to PER_SM transforms per SM while the size's plan
+// choice is the library default.  Such grids take about as long as one CTA, so
+// these plans have fewer points per thread (shorter chains, more warps to
+// share the FP64 pipe's conversions) or more registers than full SMs allow.
+template <class PL, int PER_SM>
+struct SmallBatch : PL {
+  static constexpr int SMALL_PER_SM = PER_SM;
 };
 
 // The engine a plan's kernels compute with: the fixed-point engine in the

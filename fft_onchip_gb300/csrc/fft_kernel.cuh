@@ -789,17 +789,12 @@ fft_fwd_kernel(const double2* __restrict__ in, double2* __restrict__ out, long l
       raw[i] = make_double2(__longlong_as_double(v.x), __longlong_as_double(v.y));
     }
   } else {
-    if constexpr (EK::kNatural) {
-      // threads past the batch load its last transform: no zero fill for
-      // predicated loads (2 instructions a point)
-      const double2* src = in + (TPB == 1 || active ? tr : batch - 1) * N + t;
+    // threads past the batch load its last transform: no zero fill for
+    // predicated loads (2 instructions a point at N >= 64), and no zeros, which
+    // take the general conversion (1.5 us of a single transform of 16 points)
+    const double2* src = in + (TPB == 1 || active ? tr : batch - 1) * N + t;
 #pragma unroll
-      for (int i = 0; i < P; ++i) raw[i] = load_point(src + T * i);
-    } else {
-      const double2* src = in + tr * N + t;
-#pragma unroll
-      for (int i = 0; i < P; ++i) raw[i] = active ? load_point(src + T * i) : make_double2(0.0, 0.0);
-    }
+    for (int i = 0; i < P; ++i) raw[i] = load_point(src + T * i);
   }
 
   S re[P], im[P];

@@ -37,6 +37,7 @@ struct KernelDesc {
   int prefetch = 0;          // 1: L2 prefetch one wave ahead (Prefetched<> plans)
   int code_flags = 0;        // FFTOC_CODE_* bits of the plan
   int uneven_default = 0;    // 1: the uneven path's default plan for this size (UnevenDefault<>)
+  int small_per_sm = 0;      // > 0: the default plan of batches up to this many transforms per SM (SmallBatch<>)
   // uneven-batch kernel of the same plan (nullptr for TMA-prefetching plans)
   const void* fn_uneven = nullptr;
   int smem_uneven = 0;

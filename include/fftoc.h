@@ -190,13 +190,19 @@ typedef struct {
 #define FFTOC_CODE_DIRECT_IO 8           /* small n: HBM accessed directly, no
                                             shared-memory staging of the tile */
 
-/* Plan currently used for (n, engine). */
+/* Plan currently used for (n, engine): the selected one, or while none was
+ * selected variant 0 (the batched entry points then run batches of few
+ * transforms on the plan noted at fftoc_plan_select). */
 fftoc_status fftoc_plan_query(int n, int engine, fftoc_plan_info *info);
 
 /* Any compiled plan of (n, engine), 0 <= variant < info.variants. */
 fftoc_status fftoc_plan_query_variant(int n, int engine, int variant, fftoc_plan_info *info);
 
-/* Use plan `variant` for (n, engine) from now on (process-wide).  The
+/* Use plan `variant` for (n, engine) from now on (process-wide), for every
+ * batch.  While no plan is selected, the fixed-point engine's batched entry
+ * points on device memory run batches of up to 512 (n = 8, 32, 128), 128 (16),
+ * 32 (64), 256 (256), 5 (512), 3 (1024) or 6 (2048) transforms per SM on a
+ * compiled plan with shorter chains, and larger ones on variant 0.  The
  * reference picks executor parameters (UPB, FPU) at compile time through the
  * generated sweep, scripts/generate_bench.py:93-113; here the choice is made
  * at run time among the compiled plans. */
