@@ -8,6 +8,7 @@
 // (includes/common.cuh:3-13) on any CUDA error.  This library instead returns
 // a status, keeps a per-thread message, and sizes the grid from the batch.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -282,23 +283,34 @@ fftoc_status device_plan_resources(int slot, int idx, int var, const void** tw, 
 }
 
 // Plan of a batch on device buffers: the chosen one for every batch, or while
-// none was chosen variant 0, and its SmallBatch<> plan up to that plan's limit.
-// The limits are where the two measured equal on 152 SMs, or where the larger
-// one's waves first beat it (back-to-back launches, us, variant 0 against the
-// small-batch plan, one transform and at the limit):
-//   N = 8     4.0 2.4    7.3 5.6 (77824)    256   6.2 3.5   63.6 58.8 (38912)
-//   16        2.9 2.2    3.5 3.4 (19456)    512   3.5 3.3    5.3 5.2 (760)
-//   32        4.5 2.3   15.7 15.3 (77824)   1024  4.2 3.8    6.3 6.2 (456)
-//   64        3.0 2.2    3.8 3.7 (4864)     2048  6.8 5.1   18.3 17.4 (912)
-//   128       5.6 3.5   60.2 55.8 (77824)
-// (4096: radix 8 in 512 threads 8.7 against 8.6, two barriers more: none.)
+// none was chosen the SmallBatch<> plan with the lowest limit that takes the
+// batch, else variant 0.  The limits are where two neighbours measured equal on
+// 152 SMs, or where the larger one's waves first beat the other (back-to-back
+// launches, us, variant 0 -> the plans below it, at one transform and at each
+// limit):
+//          fixed point                                 binary64
+//   8      4.0 -> 2.0   7.3 -> 5.9 (77824)             5.4 -> 2.1    6.5 -> 4.9 (29184)
+//   16     2.9 -> 2.2   3.5 -> 3.4 (19456)             3.7 -> 2.5    4.3 -> 3.6 (7296)
+//   32     4.5 -> 2.3   15.7 -> 15.3 (77824)           8.4 -> 3.1    9.0 -> 7.4 (7296)
+//   64     3.0 -> 2.2   3.8 -> 3.7 (4864)             10.1 -> 3.5   10.8 -> 8.8 (3648)
+//   128    5.6 -> 2.3   5.5 -> 3.9 (2432), 60.2 -> 55.8 (77824)   12.5 -> 4.1   13.0 -> 10.2 (1824)
+//   256    6.2 -> 2.3   6.0 -> 4.1 (1216), 63.6 -> 58.8 (38912)   14.0 -> 4.3   27.1 -> 21.8 (1824)
+//   512    3.5 -> 3.3   5.3 -> 5.2 (760)              15.0 -> 7.9   30.2 -> 26.7 (1064)
+//   1024   4.2 -> 3.8   6.3 -> 6.2 (456)              33.8 -> 15.8  132 -> 126 (2432)
+//   2048   6.8 -> 5.1   18.3 -> 17.4 (912)            radix 8 as fast: none
+//   4096   radix 8 in 512 threads 8.7 against 8.6, a barrier more: none; binary64 the same
 int batch_variant(const DeviceState& ds, int slot, int idx, int64_t batch) {
-  if (g_choice[slot][idx].load(std::memory_order_relaxed) == 0) {
-    const SizeVariants& sv = ds.var[slot][idx];
-    for (int v = 0; v < sv.count; ++v)
-      if (sv.v[v].small_per_sm > 0) return batch <= (int64_t)sv.v[v].small_per_sm * ds.sms ? v : 0;
+  if (g_choice[slot][idx].load(std::memory_order_relaxed) > 0) return chosen_variant(slot, idx);
+  const SizeVariants& sv = ds.var[slot][idx];
+  int best = 0, limit = INT_MAX;
+  for (int v = 0; v < sv.count; ++v) {
+    const int s = sv.v[v].small_per_sm;
+    if (s > 0 && s < limit && batch <= (int64_t)s * ds.sms) {
+      best = v;
+      limit = s;
+    }
   }
-  return chosen_variant(slot, idx);
+  return best;
 }
 
 // `host`: in and out are device addresses of pinned host memory (launch_fwd_host).

@@ -199,10 +199,12 @@ fftoc_status fftoc_plan_query(int n, int engine, fftoc_plan_info *info);
 fftoc_status fftoc_plan_query_variant(int n, int engine, int variant, fftoc_plan_info *info);
 
 /* Use plan `variant` for (n, engine) from now on (process-wide), for every
- * batch.  While no plan is selected, the fixed-point engine's batched entry
- * points on device memory run batches of up to 512 (n = 8, 32, 128), 128 (16),
- * 32 (64), 256 (256), 5 (512), 3 (1024) or 6 (2048) transforms per SM on a
- * compiled plan with shorter chains, and larger ones on variant 0.  The
+ * batch.  While no plan is selected, the batched entry points on device memory
+ * run batches of up to some number of transforms per SM (fixed point: 512 for
+ * n = 8, 32 and 128, 128 for 16, 32 for 64, 256 for 256, 5 for 512, 3 for 1024,
+ * 6 for 2048; binary64: 192 for 8, 48 for 16 and 32, 24 for 64, 12 for 128 and
+ * 256, 7 for 512, 16 for 1024) on compiled plans with shorter chains, and larger
+ * ones on variant 0.  The
  * reference picks executor parameters (UPB, FPU) at compile time through the
  * generated sweep, scripts/generate_bench.py:93-113; here the choice is made
  * at run time among the compiled plans. */
