@@ -234,7 +234,7 @@ fftoc_status launch_split(int n, const double* in, double* out, int64_t batch, i
   const void* bm = sd->bmat[k];
   int* err = sd->err;
   void* args[] = {(void*)&in2, (void*)&out2, (void*)&bl, (void*)&tw, (void*)&bm, (void*)&err};
-  cudaError_t e = cudaLaunchKernel(d.fn, dim3((unsigned)blocks), dim3(d.threads), args, (size_t)d.smem, stream);
+  cudaError_t e = launch_overlapped(d.fn, (unsigned)blocks, cap, d.threads, d.smem, args, stream, true);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return set_error(FFTOC_ERR_CUDA, std::string("cudaLaunchKernel(split): ") + cudaGetErrorString(e));

@@ -586,12 +586,15 @@ fft_exact_kernel(const double2* __restrict__ in, double2* __restrict__ out, long
     for (int gg = 0; gg < G; ++gg) mbar_init(bars + gg, 1);
     mbar_fence_init();
   }
+  after_previous();
+  allow_next();
+  const unsigned first = first_tile();
   // the first tile's inputs and maximum (read after the set-up barrier)
   const long long ntiles = (batch + TPB - 1) / TPB;
   int emin;        // smallest exponent field of raw
   double2 raw[8];  // the current tile's inputs, loaded during the previous tile
   {
-    const long long tr = (long long)blockIdx.x * TPB + c.j;
+    const long long tr = (long long)first * TPB + c.j;
     exact_load_inputs<T>(raw, in + (tr < batch ? tr : 0) * N + c.t + T * 8 * h, tr < batch);
     exact_transform_put<T, TPB, XP::W>(exact_high_range(raw, emin), h, c.j, c.t, red);
   }
@@ -610,7 +613,7 @@ fft_exact_kernel(const double2* __restrict__ in, double2* __restrict__ out, long
   c.tmem_rd = c.tmem + ((unsigned)((warp & 3) * 32) << 16) + 16 * h;
   c.phase = 0;
 
-  for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+  for (long long tile = first; tile < ntiles; tile += gridDim.x) {
     if (tid == 0) prefetch_next_tile<N, TPB>(in, tile, batch);
     const long long tr = tile * TPB + c.j;
     const bool active = tr < batch;

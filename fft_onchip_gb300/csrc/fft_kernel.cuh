@@ -350,6 +350,15 @@ __device__ __forceinline__ int fx_transform_max(int em, int tid, int j, int* red
 // whichever SMs have room: 9.2 instead of 5.4 us for 1/3 of a wave of N = 512).
 __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// A tile loop's first tile, as a value that exists only after
+// after_previous(): read-only loads whose addresses follow from it cannot move
+// above.  32 bits, as blockIdx is: a 64-bit value here cost the exact-slice
+// kernels 4 to 7 % at N = 128 and 512.
+__device__ __forceinline__ unsigned first_tile() {
+  unsigned t = blockIdx.x;
+  asm volatile("" : "+r"(t)::"memory");
+  return t;
+}
 // A point of the caller's input.  Not __ldg: the compiler takes read-only loads
 // as constant for the whole kernel and may move them above after_previous().
 __device__ __forceinline__ double2 load_point(const double2* p) {

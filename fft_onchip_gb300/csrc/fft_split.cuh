@@ -513,12 +513,15 @@ fft_split_kernel(const double2* __restrict__ in, double2* __restrict__ out, long
   c.t = c.tid - c.j * T;
   const int warp = c.tid >> 5;
 
-  // constant DFT-matrix slices, TMEM, mbarrier
+  // constant DFT-matrix slices, mbarrier, TMEM
   for (int i = c.tid; i < SP::B_BYTES / 16; i += SP::THREADS) reinterpret_cast<uint4*>(c.sB)[i] = __ldg(bmat + i);
   if (c.tid == 0) {
     for (int gg = 0; gg < G; ++gg) mbar_init(c.bar + gg, 1);
     mbar_fence_init();
   }
+  after_previous();
+  allow_next();
+  const unsigned first = first_tile();
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
                  "r"(SP::TMEM_COLS));
@@ -536,10 +539,10 @@ fft_split_kernel(const double2* __restrict__ in, double2* __restrict__ out, long
   const long long ntiles = (batch + TPB - 1) / TPB;
   double2 raw[16];  // the tile's points
   if constexpr (SP::LOAD_AHEAD) {
-    const long long tr = (long long)blockIdx.x * TPB + c.j;
+    const long long tr = (long long)first * TPB + c.j;
     split_load<T>(raw, in + (tr < batch ? tr : batch - 1) * N + c.t);
   }
-  for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+  for (long long tile = first; tile < ntiles; tile += gridDim.x) {
     if (c.tid == 0) prefetch_next_tile<N, TPB>(in, tile, batch);
     const long long tr = tile * TPB + c.j;
     const bool active = tr < batch;
