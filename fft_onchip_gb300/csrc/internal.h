@@ -145,12 +145,8 @@ inline cudaError_t allow_shared(const void* fn, int smem) {
 // together, so the next one's CTAs crowd on some SMs, and back to back that
 // measured up to 14 % slower at N = 256, 512, 1024 and 2048 (7-15 % faster at
 // 64, 128 and 4096); below and above the overlap wins at every N, by 3-70 %.
-// small_only: no overlap above half a wave.  For the split-form kernels, whose
-// CTAs stay for the whole grid: larger grids measured 1-2 % slower with it,
-// small ones save 2 us a call (100 transforms of 512 points: bf16x3
-// 8.2 -> 4.8 us, exact 10.3 -> 7.5 us).
 inline cudaError_t launch_overlapped(const void* fn, unsigned blocks, long long wave, int threads, int smem,
-                                     void** args, cudaStream_t stream, bool small_only = false) {
+                                     void** args, cudaStream_t stream, bool overlap = true) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3((unsigned)threads);
@@ -160,7 +156,7 @@ inline cudaError_t launch_overlapped(const void* fn, unsigned blocks, long long 
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 2LL * blocks > wave && (small_only || 25LL * blocks <= 17 * wave) ? 0 : 1;
+  cfg.numAttrs = !overlap || (2LL * blocks > wave && 25LL * blocks <= 17 * wave) ? 0 : 1;
   return cudaLaunchKernelExC(&cfg, fn, args);
 }
 

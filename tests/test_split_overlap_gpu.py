@@ -1,5 +1,6 @@
-"""Small grids of the split-form kernels, which are launched overlapped (half a
-wave and less), and the first grids above that: chains of calls against the
+"""The split-form kernels' overlapped launches: one CTA, the largest grid below
+and the first inside the sizes launched without overlap, a few tiles a CTA, and
+the first batch with too many tiles for it: chains of calls against the
 synchronised sequence, bit for bit, and under capture."""
 import pytest
 
@@ -13,7 +14,7 @@ PLANS = [("split_bf16x3", 16, 16, 2), ("split_bf16x3", 1024, 2, 4), ("split_tf32
 
 
 @pytest.mark.parametrize("engine,n,tpb,per_sm", PLANS)
-def test_small_grids(cuda, fftoc_lib, engine, n, tpb, per_sm):
-    half = cuda.cuda.get_device_properties(0).multi_processor_count * per_sm // 2
-    for ctas in (1, half, half + 1):
-        chain_in_place(cuda, fftoc_lib, n, ctas * tpb, engine)
+def test_grids(cuda, fftoc_lib, engine, n, tpb, per_sm):
+    wave = cuda.cuda.get_device_properties(0).multi_processor_count * per_sm
+    for tiles in (1, wave // 2, wave // 2 + 1, 3 * wave - 1, 16 * wave + 1):
+        chain_in_place(cuda, fftoc_lib, n, tiles * tpb, engine)
