@@ -517,23 +517,9 @@ struct Fft {
   }
 };
 
-// Where the transforms of one CTA tile live.  ContigTile: the batched entry
-// points, transform tile0 + j at element (tile0 + j) * N.  IndexedTile (the
-// uneven-batch kernel): transform j of the tile at element base[j], with the
-// bases staged in shared memory by the caller.
-template <int N>
-struct ContigTile {
-  const double2* __restrict__ in;
-  double2* __restrict__ out;
-  long long tile0, count;
-  __device__ __forceinline__ const double2* in_of(int j) const { return in + (tile0 + j) * N; }
-  __device__ __forceinline__ double2* out_of(int j) const { return out + (tile0 + j) * N; }
-  // element e of transform jj, idx = jj * N + e
-  __device__ __forceinline__ const double2* in_elem(int idx, int, int) const { return in + tile0 * N + idx; }
-  __device__ __forceinline__ double2* out_elem(int idx, int, int) const { return out + tile0 * N + idx; }
-  __device__ __forceinline__ static double2 load(const double2* p) { return __ldg(p); }
-};
-
+// Where the transforms of one CTA tile live.  IndexedTile (the uneven-batch
+// kernel): transform j of the tile at element base[j], with the bases staged in
+// shared memory by the caller.
 struct IndexedTile {
   const double2* __restrict__ in;
   double2* __restrict__ out;
@@ -733,12 +719,11 @@ __device__ __forceinline__ void fft_tile(const Tile& tl, const typename E::TW* _
 // in and out may be the same buffer (in place): a CTA reads only the tile it
 // writes, and every load of that tile (registers, or the shared staging
 // buffer) happens before its first store, which is what the __restrict__
-// qualifiers and the read-only loads rely on; the tests run every plan in
-// place.
-// Its body is fft_tile's with contiguous addressing written out: routing it
-// through fft_tile<ContigTile> computes the same results but compiled to
-// code measured 2.5-4% slower at N=64 and N=512, so the two are kept
-// separate and the tests check them against each other bit for bit.
+// qualifiers rely on; the tests run every plan in place.
+// Its body is fft_tile's with contiguous addressing written out: routed
+// through fft_tile it computes the same results but compiled to code measured
+// 2.5-4% slower at N=64 and N=512, so the two are kept separate and the tests
+// check them against each other bit for bit.
 template <class E, class PL>
 __global__ void __launch_bounds__(Fft<E, PL>::THREADS, PL::MINB)
 fft_fwd_kernel(const double2* __restrict__ in, double2* __restrict__ out, long long batch,
