@@ -242,15 +242,17 @@ fftoc_status capture_once(fftoc_uneven_plan p, bool size_nodes) {
   // its first launch
   if (size_nodes && (e = cudaGraphUpload(p->exec, p->cap)) == cudaSuccess) e = cudaStreamSynchronize(p->cap);
   if (e != cudaSuccess) return cuda_err(e, "cudaGraphUpload");
-  int tpb[kUnevenBins] = {}, wave[kUnevenBins] = {};
+  int tpb[kUnevenBins] = {}, wave[kUnevenBins] = {}, grid[kUnevenBins] = {};
   for (int i = 0; i < kNumSizes; ++i) {
     tpb[i] = p->kd[i]->tpb;
     wave[i] = (int)wave_blocks(p, i);
+    grid[i] = (int)persistent_blocks(p, i);
   }
   char* a = reinterpret_cast<char*>(p->args);
   if ((e = cudaMemcpy(a + offsetof(UnevenArgs, nodes), nodes, sizeof(nodes), cudaMemcpyHostToDevice)) != cudaSuccess ||
       (e = cudaMemcpy(a + offsetof(UnevenArgs, tpb), tpb, sizeof(tpb), cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaMemcpy(a + offsetof(UnevenArgs, wave), wave, sizeof(wave), cudaMemcpyHostToDevice)) != cudaSuccess)
+      (e = cudaMemcpy(a + offsetof(UnevenArgs, wave), wave, sizeof(wave), cudaMemcpyHostToDevice)) != cudaSuccess ||
+      (e = cudaMemcpy(a + offsetof(UnevenArgs, grid), grid, sizeof(grid), cudaMemcpyHostToDevice)) != cudaSuccess)
     return cuda_err(e, "cudaMemcpy(uneven graph nodes)");
   p->device_sized = size_nodes;
   return FFTOC_OK;
