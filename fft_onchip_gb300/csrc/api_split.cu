@@ -130,10 +130,15 @@ void setup(SplitDevice& sd, int dev) {
         sd.error = "split matrix size mismatch";
         return;
       }
-      if ((e = cudaFuncSetAttribute(d.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem)) != cudaSuccess)
-        return bad(e, "cudaFuncSetAttribute(split)");
-      if ((e = fit_carveout(d.fn, d.threads, d.smem, &d.blocks_per_sm)) != cudaSuccess)
-        return bad(e, "occupancy / carveout (split)");
+      int per_sm[2];
+      for (int v = 0; v < 2; ++v) {
+        const void* fn = v == 0 ? d.fn : d.fn_overlap;
+        if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem)) != cudaSuccess)
+          return bad(e, "cudaFuncSetAttribute(split)");
+        if ((e = fit_carveout(fn, d.threads, d.smem, &per_sm[v])) != cudaSuccess)
+          return bad(e, "occupancy / carveout (split)");
+      }
+      d.blocks_per_sm = per_sm[0] < per_sm[1] ? per_sm[0] : per_sm[1];
       KernelDesc kd;
       kd.passes = d.passes;
       for (int r = 0; r < 4; ++r) kd.radix[r] = d.radix[r];
@@ -151,6 +156,7 @@ void setup(SplitDevice& sd, int dev) {
         bytes = fx.size() * 4;
       } else {
         for (size_t q = 0; q < f64.size(); ++q) f32[q] = (float)f64[q];
+        if (f32.size() < 4 * (size_t)kSizes[i]) f32.resize(4 * (size_t)kSizes[i], 0.f);  // room for N points
         src = f32.data();
         bytes = f32.size() * 4;
       }
@@ -239,7 +245,7 @@ fftoc_status launch_split(int n, const double* in, double* out, int64_t batch, i
   // 8.2 -> 4.8, 912 of 1024 11.8 -> 8.7, 2432 of 4096 89.8 -> 87.8; exact, 608
   // of 1024 14.4 -> 11.5), those of 32 tiles a CTA lose 1 to 2 %.
   const bool overlap = tiles <= 16 * cap;
-  cudaError_t e = launch_overlapped(d.fn, (unsigned)blocks, cap, d.threads, d.smem, args, stream, overlap);
+  cudaError_t e = launch_overlapped(overlap ? d.fn_overlap : d.fn, (unsigned)blocks, cap, d.threads, d.smem, args, stream, overlap);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return set_error(FFTOC_ERR_CUDA, std::string("cudaLaunchKernel(split): ") + cudaGetErrorString(e));

@@ -264,10 +264,10 @@ struct ExactCtx {
 };
 
 // A thread's 8 inputs of a tile (zeros past the batch).
-template <int T>
+template <int T, bool OVERLAP>
 __device__ __forceinline__ void exact_load_inputs(double2 (&raw)[8], const double2* src, bool active) {
 #pragma unroll
-  for (int i = 0; i < 8; ++i) raw[i] = active ? __ldg(src + T * i) : make_double2(0.0, 0.0);
+  for (int i = 0; i < 8; ++i) raw[i] = active ? split_point<OVERLAP>(src + T * i) : make_double2(0.0, 0.0);
 }
 
 // Passes whose twiddles are loaded into registers before the barrier that
@@ -352,7 +352,7 @@ __device__ __forceinline__ void exact_small_dfts(long long (&re)[8], long long (
 // last pass loads the next tile's inputs into `raw` (at its start, or for a
 // radix-16 last pass once its digits are stored) so that their latency
 // overlaps the pass.
-template <class PL, int G, int s>
+template <class PL, int G, int s, bool OVERLAP>
 __device__ __forceinline__ void exact_pass(ExactCtx& c, long long (&re)[8], long long (&im)[8], const ExactOut& o,
                                            double2 (&raw)[8], const int4 (&w)[8], const int2 (&ws)[8]) {
   using XP = ExactPlan<PL, G>;
@@ -406,7 +406,7 @@ __device__ __forceinline__ void exact_pass(ExactCtx& c, long long (&re)[8], long
       for (int b = 0; b < kExactBlocks; ++b)
         *reinterpret_cast<uint4*>(c.sA + b * XP::A_BLOCK + off) = make_uint4(w[b][0], w[b][1], w[b][2], w[b][3]);
     }
-    if constexpr (s == NS - 1) exact_load_inputs<T>(raw, c.nsrc, c.nactive);
+    if constexpr (s == NS - 1) exact_load_inputs<T, OVERLAP>(raw, c.nsrc, c.nactive);
     exact_tmem_fill(c.tmem_rd);
     fence_proxy_async_smem();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -457,7 +457,7 @@ __device__ __forceinline__ void exact_pass(ExactCtx& c, long long (&re)[8], long
     }
   } else {
     // last pass of radix 2/4/8 on the CUDA cores, fixed point
-    exact_load_inputs<T>(raw, c.nsrc, c.nactive);
+    exact_load_inputs<T, OVERLAP>(raw, c.nsrc, c.nactive);
     constexpr int Bq = 16 / R, Bh = Bq / 2;
 #pragma unroll
     for (int b = 0; b < Bh; ++b)
@@ -497,7 +497,7 @@ __device__ __forceinline__ void exact_pass(ExactCtx& c, long long (&re)[8], long
     if constexpr (EARLY_SMALL_TW<PL, s + 1>) exact_load_small_twiddles<PL, s + 1>(c, wn, wsn);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    exact_pass<PL, G, s + 1>(c, re, im, o, raw, wn, wsn);
+    exact_pass<PL, G, s + 1, OVERLAP>(c, re, im, o, raw, wn, wsn);
   }
 }
 
@@ -548,7 +548,7 @@ __device__ __forceinline__ unsigned exact_transform_get(int j, const unsigned* r
   return a;
 }
 
-template <class PL, int G>
+template <class PL, int G, bool OVERLAP>
 __global__ void __launch_bounds__(256 * G, G == 1 ? 2 : 1)
 fft_exact_kernel(const double2* __restrict__ in, double2* __restrict__ out, long long batch,
                  const int4* __restrict__ tw, const uint4* __restrict__ bmat, int* __restrict__ err) {
@@ -595,7 +595,7 @@ fft_exact_kernel(const double2* __restrict__ in, double2* __restrict__ out, long
   double2 raw[8];  // the current tile's inputs, loaded during the previous tile
   {
     const long long tr = (long long)first * TPB + c.j;
-    exact_load_inputs<T>(raw, in + (tr < batch ? tr : 0) * N + c.t + T * 8 * h, tr < batch);
+    exact_load_inputs<T, OVERLAP>(raw, in + (tr < batch ? tr : 0) * N + c.t + T * 8 * h, tr < batch);
     exact_transform_put<T, TPB, XP::W>(exact_high_range(raw, emin), h, c.j, c.t, red);
   }
   if (warp == 0) {
@@ -645,7 +645,7 @@ fft_exact_kernel(const double2* __restrict__ in, double2* __restrict__ out, long
                      (int)((unsigned)k_out << 20), k_out};
     const int4 w0[8] = {};
     const int2 ws0[8] = {};
-    exact_pass<PL, G, 0>(c, re, im, o, raw, w0, ws0);
+    exact_pass<PL, G, 0, OVERLAP>(c, re, im, o, raw, w0, ws0);
     // the next tile's maximum, read after the barrier
     exact_transform_put<T, TPB, XP::W>(exact_high_range(raw, emin), h, c.j, c.t, red);
     if (__syncthreads_or(c.failed)) {

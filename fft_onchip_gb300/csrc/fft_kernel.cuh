@@ -359,8 +359,11 @@ __device__ __forceinline__ unsigned first_tile() {
   asm volatile("" : "+r"(t)::"memory");
   return t;
 }
-// A point of the caller's input.  Not __ldg: the compiler takes read-only loads
-// as constant for the whole kernel and may move them above after_previous().
+// A point of the caller's input.  Not __ldg: a kernel launched with the overlap
+// is there while the one before it still writes this memory, and a read-only
+// load is defined only where nothing writes during the kernel's lifetime (the
+// compiler may move it above after_previous(), and a line that it left in L1
+// need not be dropped by the wait).
 __device__ __forceinline__ double2 load_point(const double2* p) {
   double2 v;
   asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));

@@ -316,7 +316,7 @@ __device__ __noinline__ void split_unscale_outputs(double2* dst, int t, int unsh
 // A point again, scaled by 2^shift (exact, binary64) before the general
 // conversion: transforms out of the FP32 range or not finite.  Out of line.
 __device__ __noinline__ float2 split_reload(const double2* p, int shift) {
-  const double2 v = *p;
+  const double2 v = load_point(p);
   return make_float2(f64_to_f32_int(ldexp(v.x, shift)), f64_to_f32_int(ldexp(v.y, shift)));
 }
 
@@ -330,14 +330,30 @@ struct SplitCtx {
   unsigned tmem, idesc, phase;
   int tid, g, row, lane_block, j, t;
   bool failed;  // a bounded wait gave up (the tile loop ends after the tile)
-  const double2* nsrc;  // this thread's first point of the next tile
+  // this thread's first point of the next tile; after the last one, of N points
+  // of the twiddle table's allocation: what is left of the batch belongs to other
+  // CTAs, which may be storing it, and a branch around the loads, or zeros in
+  // their place, made the kernels 2 to 20 % slower at half of the sizes
+  const double2* nsrc;
 };
 
+// A point of the caller's input in the split forms, whose CTAs live as long as
+// the grid.  OVERLAP: the kernel of overlapped launches (load_point).  The other
+// one has the device to itself while the input is read, and read-only loads,
+// which may be scheduled across its barriers (1 GiB, against load_point: BF16x3
+// and TF32x2 4 % faster at N = 32, 0 to 2 % elsewhere; exact slices 10 % at
+// N = 128, 595 against 653 us, 1 to 4 % at 32, 64, 512 and 1024).
+template <bool OVERLAP>
+__device__ __forceinline__ double2 split_point(const double2* p) {
+  if constexpr (OVERLAP) return load_point(p);
+  else return __ldg(p);
+}
+
 // A thread's 16 points of a tile.
-template <int T>
+template <int T, bool OVERLAP>
 __device__ __forceinline__ void split_load(double2 (&raw)[16], const double2* src) {
 #pragma unroll
-  for (int i = 0; i < 16; ++i) raw[i] = __ldg(src + T * i);
+  for (int i = 0; i < 16; ++i) raw[i] = split_point<OVERLAP>(src + T * i);
 }
 
 // Barrier over the threads that share data inside a tile: the thread's
@@ -357,7 +373,7 @@ __device__ __forceinline__ void tile_sync(int g) {
 // `dst` (transform base, binary64).  A bounded wait that gives up sets
 // c.failed; the passes still run their barriers so every thread reaches the
 // end of the tile.
-template <int KIND, class PL, int G, int s>
+template <int KIND, class PL, int G, int s, bool OVERLAP>
 __device__ __forceinline__ void split_pass(SplitCtx& c, float (&re)[16], float (&im)[16], double2* dst, bool active,
                                            int unshift, bool scaled, bool special, double2 (&raw)[16]) {
   using SP = SplitPlan<KIND, PL, G>;
@@ -411,7 +427,7 @@ __device__ __forceinline__ void split_pass(SplitCtx& c, float (&re)[16], float (
                    : "memory");
     }
     // the next tile's points, while the MMAs run and the thread's own are gone
-    if constexpr (s == NS - 1 && SP::LOAD_AHEAD) split_load<T>(raw, c.nsrc);
+    if constexpr (s == NS - 1 && SP::LOAD_AHEAD) split_load<T, OVERLAP>(raw, c.nsrc);
     if (!c.failed && !mbar_wait_bounded(c.bar + c.g, c.phase, kWaitLimitNs)) c.failed = true;
     c.phase ^= 1;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -424,7 +440,7 @@ __device__ __forceinline__ void split_pass(SplitCtx& c, float (&re)[16], float (
     }
   } else {
     // last pass of radix 2/4/8 on the CUDA cores: 16/R butterflies per thread
-    split_load<T>(raw, c.nsrc);
+    split_load<T, OVERLAP>(raw, c.nsrc);
 #pragma unroll
     for (int b = 0; b < Bq; ++b) {
       const int tp = c.t + T * b;
@@ -452,7 +468,7 @@ __device__ __forceinline__ void split_pass(SplitCtx& c, float (&re)[16], float (
       }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");  // this pass's TMEM reads precede the next MMAs
     tile_sync<SP::GROUP_LOCAL>(c.g);
-    split_pass<KIND, PL, G, s + 1>(c, re, im, dst, active, unshift, scaled, special, raw);
+    split_pass<KIND, PL, G, s + 1, OVERLAP>(c, re, im, dst, active, unshift, scaled, special, raw);
   } else {
     if (active) {
       // zeros (and subnormals) and non-finite transforms take the general
@@ -488,7 +504,8 @@ __device__ __forceinline__ void split_pass(SplitCtx& c, float (&re)[16], float (
   }
 }
 
-template <int KIND, class PL, int G>
+// tw: the twiddles, in an allocation of at least N points (SplitCtx::nsrc).
+template <int KIND, class PL, int G, bool OVERLAP>
 __global__ void __launch_bounds__(128 * G, PL::MINB)
 fft_split_kernel(const double2* __restrict__ in, double2* __restrict__ out, long long batch,
                  const float2* __restrict__ tw, const uint4* __restrict__ bmat, int* __restrict__ err) {
@@ -537,10 +554,12 @@ fft_split_kernel(const double2* __restrict__ in, double2* __restrict__ out, long
   c.failed = false;
 
   const long long ntiles = (batch + TPB - 1) / TPB;
-  double2 raw[16];  // the tile's points
+  // the tile's points; in the last tile, rows past the batch compute with its
+  // first transform (zeros without the loads ahead)
+  double2 raw[16];
   if constexpr (SP::LOAD_AHEAD) {
     const long long tr = (long long)first * TPB + c.j;
-    split_load<T>(raw, in + (tr < batch ? tr : batch - 1) * N + c.t);
+    split_load<T, OVERLAP>(raw, in + (tr < batch ? tr : (long long)first * TPB) * N + c.t);
   }
   for (long long tile = first; tile < ntiles; tile += gridDim.x) {
     if (c.tid == 0) prefetch_next_tile<N, TPB>(in, tile, batch);
@@ -549,10 +568,13 @@ fft_split_kernel(const double2* __restrict__ in, double2* __restrict__ out, long
     // ---- load and convert: point i of this thread is element t + T*i;
     // per-transform power-of-two scale when the largest magnitude is outside
     // [2^-60, 2^60]
-    const double2* src = in + (active ? tr : batch - 1) * N + c.t;
-    const long long ntr = tr + (long long)gridDim.x * TPB;
-    c.nsrc = in + (ntr < batch ? ntr : batch - 1) * N + c.t;
-    if constexpr (!SP::LOAD_AHEAD) split_load<T>(raw, src);
+    const double2* src = in + tr * N + c.t;  // only read where active
+    const long long next = (tile + gridDim.x) * TPB, ntr = next + c.j;
+    c.nsrc = (next < batch ? in + (ntr < batch ? ntr : next) * N : reinterpret_cast<const double2*>(tw)) + c.t;
+    if constexpr (!SP::LOAD_AHEAD) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) raw[i] = active ? split_point<OVERLAP>(src + T * i) : make_double2(0.0, 0.0);
+    }
     float re[16], im[16];
     int em, emin;
     fx_exponent_range<16>(raw, em, emin);
@@ -567,7 +589,7 @@ fft_split_kernel(const double2* __restrict__ in, double2* __restrict__ out, long
     const bool scaled = em < 2047 && (em > 1023 + 60 || em < 1023 - 60);
     const int shift = scaled ? (em == 0 ? 1023 + 52 : 1023 - em) : 0;
     const bool special = em == 2047;
-    if (scaled || special) {  // rare
+    if (active && (scaled || special)) {  // rare
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const float2 v = split_reload(src + T * i, shift);
@@ -575,7 +597,7 @@ fft_split_kernel(const double2* __restrict__ in, double2* __restrict__ out, long
         im[i] = v.y;
       }
     }
-    split_pass<KIND, PL, G, 0>(c, re, im, out + tr * N, active, -shift, scaled, special, raw);
+    split_pass<KIND, PL, G, 0, OVERLAP>(c, re, im, out + tr * N, active, -shift, scaled, special, raw);
     // exchange buffer and exponent scratch free for the next tile; stop after
     // a bounded wait gave up anywhere in the CTA
     if (__syncthreads_or(c.failed)) {

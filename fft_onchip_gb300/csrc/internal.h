@@ -66,7 +66,8 @@ void describe_onchip_fx(SizeVariants* per_size);
 
 // Split-precision form: one compiled plan per size (fn == nullptr: none).
 struct SplitDesc {
-  const void* fn = nullptr;
+  const void* fn = nullptr;          // the kernel of plain launches
+  const void* fn_overlap = nullptr;  // and of overlapped ones (launch_overlapped)
   int threads = 0, tpb = 0, smem = 0, passes = 0;
   int radix[4] = {1, 1, 1, 1};
   int tw_entries = 0;  // FP32 twiddles (8 bytes each)

@@ -15,7 +15,8 @@ namespace {
 template <int KIND, class PL, int G>
 void add_split(SplitDesc& d) {
   using SP = SplitPlan<KIND, PL, G>;
-  d.fn = (const void*)&fft_split_kernel<KIND, PL, G>;
+  d.fn = (const void*)&fft_split_kernel<KIND, PL, G, false>;
+  d.fn_overlap = (const void*)&fft_split_kernel<KIND, PL, G, true>;
   d.threads = SP::THREADS;
   d.tpb = PL::TPB;
   d.smem = SP::SMEM;
@@ -46,7 +47,8 @@ void describe(SplitDesc* d) {
 template <class PL, int G>
 void add_exact(SplitDesc& d) {
   using XP = ExactPlan<PL, G>;
-  d.fn = (const void*)&fft_exact_kernel<PL, G>;
+  d.fn = (const void*)&fft_exact_kernel<PL, G, false>;
+  d.fn_overlap = (const void*)&fft_exact_kernel<PL, G, true>;
   d.threads = XP::THREADS;
   d.tpb = PL::TPB;
   d.smem = XP::SMEM;
