@@ -17,8 +17,11 @@
 #include <string>
 #include <vector>
 
+#include <cuda.h>
+
 #include "../../include/fftoc.h"
 #include "fft_core.cuh"
+#include "host_range.h"
 #include "internal.h"
 
 namespace fftoc {
@@ -365,20 +368,44 @@ fftoc_status launch_fwd(int n, const double* in, double* out, int64_t batch, int
 // against 810).
 constexpr uintptr_t kDirectIoHostBytes = (uintptr_t)128 << 20;
 
+// cuPointerGetAttributes, or null (a driver without it: host buffers are staged).
+using PointerAttributes = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+PointerAttributes pointer_attributes() {
+  static const PointerAttributes fn = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault, &found) != cudaSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return found == cudaDriverEntryPointSuccess ? reinterpret_cast<PointerAttributes>(f) : nullptr;
+  }();
+  return fn;
+}
+
 // The device address of `bytes` of host memory at p if all of it is pinned and
-// mapped (its first and last points are, at one distance from their addresses),
-// else null.
+// mapped, else null.  By the registrations' ranges: under unified addressing
+// the device addresses of a buffer's two ends say nothing of what lies between.
 void* mapped_host(const void* p, size_t bytes) {
-  cudaPointerAttributes a, b;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess ||
-      cudaPointerGetAttributes(&b, static_cast<const char*>(p) + bytes - 16) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer || !b.devicePointer) return nullptr;
-  return static_cast<char*>(b.devicePointer) - static_cast<char*>(a.devicePointer) == (ptrdiff_t)(bytes - 16)
-             ? a.devicePointer
-             : nullptr;
+  const PointerAttributes get = pointer_attributes();
+  if (!get) return nullptr;
+  return mapped_range(p, bytes, [&](uintptr_t at) {
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                  CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    unsigned type = 0, managed = 0;
+    CUdeviceptr dev = 0, start = 0;
+    size_t size = 0;
+    void* to[] = {&type, &managed, &dev, &start, &size};
+    HostRange r = {};
+    if (get(5, what, to, (CUdeviceptr)at) != CUDA_SUCCESS) return r;
+    // the range's start is the host's address or the device's
+    const ptrdiff_t shift = (ptrdiff_t)(dev - (CUdeviceptr)at);
+    if (type != CU_MEMORYTYPE_HOST || managed || !dev || size == 0) return r;
+    const uintptr_t host = at - start < size ? (uintptr_t)start : (uintptr_t)start - (uintptr_t)shift;
+    r = {true, host, size, shift};
+    return r;
+  });
 }
 
 // Host buffers.  The binary64 and fixed-point engines transform pinned memory
