@@ -13,11 +13,11 @@ tensor, forward (exp(-2*pi*i*n*k/N)), unnormalised, natural order, like
 (includes/testing.cuh:16-57).
 """
 from ._lib import (ENGINE_AUTO, ENGINE_DMMA, ENGINE_F64, ENGINE_FX, ENGINE_SPLIT_BF16X3, ENGINE_SPLIT_EXACT,
-                   ENGINE_SPLIT_TF32X2, ENGINES, EXPORTS, SIZES, FftocError, autotune, check, load, plan_query,
-                   plan_select)
+                   ENGINE_SPLIT_TF32X2, ENGINES, EXPORTS, SIZES, FftocError, autotune, check, load,
+                   plan_for_batch, plan_query, plan_restore, plan_select, plan_selected)
 
-__all__ = ["fft", "fft_ptr", "fft_host", "fft_host_ptr", "plan_query", "plan_select", "autotune", "FftocError", "SIZES",
-           "ENGINES", "load", "auto_engine", "UnevenPlan", "fft_uneven"]
+__all__ = ["fft", "fft_ptr", "fft_host", "fft_host_ptr", "plan_query", "plan_for_batch", "plan_select", "plan_selected",
+           "plan_restore", "autotune", "FftocError", "SIZES", "ENGINES", "load", "auto_engine", "UnevenPlan", "fft_uneven"]
 
 
 def _engine_id(engine):

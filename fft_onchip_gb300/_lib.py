@@ -39,7 +39,10 @@ EXPORTS = tuple(["fftoc_c2c_fwd_n%d" % n for n in SIZES]) + (
     "fftoc_c2c_fwd_split",
     "fftoc_plan_query",
     "fftoc_plan_query_variant",
+    "fftoc_plan_query_batch",
     "fftoc_plan_select",
+    "fftoc_plan_selected",
+    "fftoc_plan_unselect",
     "fftoc_autotune",
     "fftoc_device_error_check",
     "fftoc_auto_engine",
@@ -148,8 +151,14 @@ def load(path=None):
     L.fftoc_plan_query.restype = c_int
     L.fftoc_plan_query_variant.argtypes = [c_int, c_int, c_int, ctypes.POINTER(PlanInfo)]
     L.fftoc_plan_query_variant.restype = c_int
+    L.fftoc_plan_query_batch.argtypes = [c_int, c_int, i64, c_int, ctypes.POINTER(PlanInfo)]
+    L.fftoc_plan_query_batch.restype = c_int
     L.fftoc_plan_select.argtypes = [c_int, c_int, c_int]
     L.fftoc_plan_select.restype = c_int
+    L.fftoc_plan_selected.argtypes = [c_int, c_int, ctypes.POINTER(c_int)]
+    L.fftoc_plan_selected.restype = c_int
+    L.fftoc_plan_unselect.argtypes = [c_int, c_int]
+    L.fftoc_plan_unselect.restype = c_int
     L.fftoc_autotune.argtypes = [c_int, c_int, i64, vp, ctypes.POINTER(c_int), ctypes.POINTER(ctypes.c_float)]
     L.fftoc_autotune.restype = c_int
     L.fftoc_device_error_check.argtypes = []
@@ -242,8 +251,30 @@ def plan_query(n, engine=ENGINE_AUTO, variant=None):
     return _info_dict(info)
 
 
+def plan_for_batch(n, engine, batch, sms):
+    """Plan of a call on `batch` transforms on a device of `sms` multiprocessors."""
+    info = PlanInfo()
+    check(load().fftoc_plan_query_batch(int(n), int(engine), int(batch), int(sms), ctypes.byref(info)))
+    return _info_dict(info)
+
+
 def plan_select(n, engine, variant):
     check(load().fftoc_plan_select(int(n), int(engine), int(variant)))
+
+
+def plan_selected(n, engine):
+    """The selected variant of (n, engine), or None while none is."""
+    v = ctypes.c_int()
+    check(load().fftoc_plan_selected(int(n), int(engine), ctypes.byref(v)))
+    return None if v.value < 0 else v.value
+
+
+def plan_restore(n, engine, selected):
+    """Put back what plan_selected returned."""
+    if selected is None:
+        check(load().fftoc_plan_unselect(int(n), int(engine)))
+    else:
+        plan_select(n, engine, selected)
 
 
 def autotune(n, engine, batch, stream_ptr=0):

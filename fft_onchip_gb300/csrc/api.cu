@@ -107,7 +107,8 @@ struct DeviceState {
 };
 
 // Plan chosen per (engine, size), plus one: process-wide, set by
-// fftoc_plan_select or fftoc_autotune; 0 until then.
+// fftoc_plan_select or fftoc_autotune; 0 until then and after
+// fftoc_plan_unselect.
 std::atomic<int> g_choice[2][kNumSizes];
 
 const SizeVariants* host_variants(int eng_slot) {
@@ -285,8 +286,8 @@ fftoc_status device_plan_resources(int slot, int idx, int var, const void** tw, 
   return FFTOC_OK;
 }
 
-// Plan of a batch on device buffers: the chosen one for every batch, or while
-// none was chosen the SmallBatch<> plan with the lowest limit that takes the
+// Plan of a batch, on device buffers and on host buffers (which give the same
+// bits therefore): the chosen one for every batch, or while none was chosen the SmallBatch<> plan with the lowest limit that takes the
 // batch, else variant 0.  The limits are where two neighbours measured equal on
 // 152 SMs, or where the larger one's waves first beat the other (back-to-back
 // launches, us, variant 0 -> the plans below it, at one transform and at each
@@ -302,13 +303,14 @@ fftoc_status device_plan_resources(int slot, int idx, int var, const void** tw, 
 //   1024   4.2 -> 3.8   6.3 -> 6.2 (456)              33.8 -> 15.8  132 -> 126 (2432)
 //   2048   6.8 -> 5.1   18.3 -> 17.4 (912)            radix 8 as fast: none
 //   4096   radix 8 in 512 threads 8.7 against 8.6, a barrier more: none; binary64 the same
-int batch_variant(const DeviceState& ds, int slot, int idx, int64_t batch) {
-  if (g_choice[slot][idx].load(std::memory_order_relaxed) > 0) return chosen_variant(slot, idx);
-  const SizeVariants& sv = ds.var[slot][idx];
+int batch_variant(int slot, int idx, int64_t batch, int sms) {
+  const int c = g_choice[slot][idx].load(std::memory_order_relaxed);
+  if (c > 0) return c - 1;
+  const SizeVariants& sv = host_variants(slot)[idx];
   int best = 0, limit = INT_MAX;
   for (int v = 0; v < sv.count; ++v) {
     const int s = sv.v[v].small_per_sm;
-    if (s > 0 && s < limit && batch <= (int64_t)s * ds.sms) {
+    if (s > 0 && s < limit && batch <= (int64_t)s * sms) {
       best = v;
       limit = s;
     }
@@ -341,13 +343,18 @@ fftoc_status launch_fwd(int n, const double* in, double* out, int64_t batch, int
   fftoc_status st = device_state(&ds);
   if (st != FFTOC_OK) return st;
   const int slot = eng == FFTOC_ENGINE_FX ? 1 : 0;
-  const int var = variant >= 0 ? variant : batch_variant(*ds, slot, idx, batch);
+  const int var = variant >= 0 ? variant : batch_variant(slot, idx, batch, ds->sms);
   if (var >= ds->var[slot][idx].count) return fail(FFTOC_ERR_INVALID_VALUE, "no such plan variant");
   const KernelDesc& d = ds->var[slot][idx].v[var];
   const void* tw = ds->tw[slot][idx][var];
   const long long tiles = (batch + d.tpb - 1) / d.tpb;
-  const int smem = host && d.smem < kDirectSmem ? kDirectSmem : d.smem;
-  const long long cap = (long long)ds->sms * (smem > d.smem ? 1 : d.blocks_per_sm);
+  // host buffers: as many CTAs per SM as hold 8 KB of tiles (launch_fwd_host)
+  int smem = d.smem, per_sm = d.blocks_per_sm;
+  if (host) {
+    const int want = d.tpb * n * 16 >= 8192 ? 1 : 8192 / (d.tpb * n * 16), alone = direct_smem(want);
+    if (alone > smem) smem = alone, per_sm = want;
+  }
+  const long long cap = (long long)ds->sms * per_sm;
   const long long blocks = d.persistent ? (tiles < cap ? tiles : cap) : tiles;
   if (blocks > 0x7FFFFFFFLL) return fail(FFTOC_ERR_INVALID_VALUE, "batch too large for one launch");
   const double2* in2 = reinterpret_cast<const double2*>(in);
@@ -410,13 +417,15 @@ void* mapped_host(const void* p, size_t bytes) {
 
 // Host buffers.  The binary64 and fixed-point engines transform pinned memory
 // in place of it: one launch whose CTAs load their tile over the host link and
-// store the result over it.  One CTA per SM (kDirectSmem) keeps 2-10 MB in
-// flight, enough for the link's latency; with full occupancy the first wave
-// only reads and the last only writes, 20-80 MB each.  Measured on one GB300
-// against staging (which pays the copies' launches, and a chunk each way
-// outside the overlap), n = 256: 10 KB 15 us against 33, 4 MB 47 against 71, 82 MB 513 against 812, 1 GB
-// 6.0 ms against 6.5 (164-171 GB/s each way, the link's rate in both directions
-// at once).  Pageable memory and the other engines are staged.
+// store the result over it.  One CTA per SM, or as many as hold 8 KB of tiles
+// (direct_smem), keep 1.2 to 10 MB in flight, enough for the link's latency: 82 MB
+// take 503 us in tiles of 8 KB (N = 64, 128, 256 and 512; 163 GB/s each way, the
+// link's rate in both directions at once), 510 to 600 us in 16 to 64 KB (N = 1024,
+// 2048 and 4096).  With full occupancy the first wave only reads and the last
+// only writes, 20-80 MB each.  Against staging (which pays the copies' launches,
+// and a chunk each way outside the overlap), n = 256: 10 KB 19 us against 33,
+// 4 MB 45 against 71, 82 MB 504 against 812, 1 GB 6.0 ms against 6.5.  Pageable
+// memory and the other engines are staged.
 fftoc_status launch_fwd_host(int n, const double* h_in, double* h_out, int64_t batch, int engine,
                              cudaStream_t stream) {
   const int idx = size_index(n);
@@ -437,10 +446,9 @@ fftoc_status launch_fwd_host(int n, const double* h_in, double* h_out, int64_t b
   if (d_in && h_out != h_in) d_out = mapped_host(h_out, bytes);
   const int eng = resolve_engine(n, engine);
   const int slot = eng == FFTOC_ENGINE_FX ? 1 : 0;
-  // one plan for the whole call, and not the small-batch one: the link bounds
-  // these, and the larger tiles keep more of it in flight
+  // the plan of a device batch of this count, for every chunk
   const bool planned = eng == FFTOC_ENGINE_FX || eng == FFTOC_ENGINE_F64;
-  const int var = planned ? chosen_variant(slot, idx) : -1;
+  const int var = planned ? batch_variant(slot, idx, batch, ds->sms) : -1;
   const KernelDesc& plan = ds->var[slot][idx].v[planned ? var : 0];
   if (d_in && d_out && planned &&
       !plan.persistent &&  // bulk copies stay on device memory
@@ -486,7 +494,8 @@ fftoc_status launch_fwd_host(int n, const double* h_in, double* h_out, int64_t b
   return FFTOC_OK;
 }
 
-fftoc_status plan_query(int n, int engine, int variant, fftoc_plan_info* info) {
+// variant < 0: the plan in use, for a batch of `batch` on `sms` SMs if batch >= 0.
+fftoc_status plan_query(int n, int engine, int variant, fftoc_plan_info* info, int64_t batch = -1, int sms = 0) {
   const int idx = size_index(n);
   if (idx < 0) return fail(FFTOC_ERR_INVALID_SIZE, "n=" + std::to_string(n) + " is not one of 8,16,...,4096");
   if (!info) return fail(FFTOC_ERR_INVALID_VALUE, "null info");
@@ -504,7 +513,7 @@ fftoc_status plan_query(int n, int engine, int variant, fftoc_plan_info* info) {
   }
   const int slot = eng == FFTOC_ENGINE_FX ? 1 : 0;
   const SizeVariants& sv = host_variants(slot)[idx];
-  const int var = variant >= 0 ? variant : chosen_variant(slot, idx);
+  const int var = variant >= 0 ? variant : batch >= 0 ? batch_variant(slot, idx, batch, sms) : chosen_variant(slot, idx);
   if (var >= sv.count) return fail(FFTOC_ERR_INVALID_VALUE, "no such plan variant");
   const KernelDesc& d = sv.v[var];
   info->n = n;
@@ -565,6 +574,31 @@ fftoc_status plan_select(int n, int engine, int variant) {
   if (info.engine == FFTOC_ENGINE_FX || info.engine == FFTOC_ENGINE_F64)
     g_choice[info.engine == FFTOC_ENGINE_FX ? 1 : 0][size_index(n)].store(variant + 1);
   return FFTOC_OK;
+}
+
+// The stored choice of (n, engine), or null for an engine with one plan a size.
+fftoc_status plan_choice(int n, int engine, std::atomic<int>** choice) {
+  fftoc_plan_info info;
+  const fftoc_status st = plan_query(n, engine, 0, &info);
+  *choice = nullptr;
+  if (st == FFTOC_OK && (info.engine == FFTOC_ENGINE_FX || info.engine == FFTOC_ENGINE_F64))
+    *choice = &g_choice[info.engine == FFTOC_ENGINE_FX ? 1 : 0][size_index(n)];
+  return st;
+}
+
+fftoc_status plan_selected(int n, int engine, int* variant) {
+  if (!variant) return fail(FFTOC_ERR_INVALID_VALUE, "null variant");
+  std::atomic<int>* c;
+  const fftoc_status st = plan_choice(n, engine, &c);
+  if (st == FFTOC_OK) *variant = c ? c->load() - 1 : -1;
+  return st;
+}
+
+fftoc_status plan_unselect(int n, int engine) {
+  std::atomic<int>* c;
+  const fftoc_status st = plan_choice(n, engine, &c);
+  if (c) c->store(0);
+  return st;
 }
 
 // Time every compiled plan of (n, engine) on a device scratch batch of
@@ -659,7 +693,16 @@ fftoc_status fftoc_plan_query_variant(int n, int engine, int variant, fftoc_plan
   return fftoc::plan_query(n, engine, variant, info);
 }
 
+fftoc_status fftoc_plan_query_batch(int n, int engine, int64_t batch, int sms, fftoc_plan_info* info) {
+  if (batch < 0 || sms < 1) return fftoc::fail(FFTOC_ERR_INVALID_VALUE, "batch must be >= 0 and sms >= 1");
+  return fftoc::plan_query(n, engine, -1, info, batch, sms);
+}
+
 fftoc_status fftoc_plan_select(int n, int engine, int variant) { return fftoc::plan_select(n, engine, variant); }
+
+fftoc_status fftoc_plan_selected(int n, int engine, int* variant) { return fftoc::plan_selected(n, engine, variant); }
+
+fftoc_status fftoc_plan_unselect(int n, int engine) { return fftoc::plan_unselect(n, engine); }
 
 fftoc_status fftoc_device_error_check(void) { return fftoc::device_error_check(); }
 

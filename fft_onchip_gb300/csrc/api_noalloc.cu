@@ -163,7 +163,7 @@ fftoc_status launch_fwd_host_noalloc(int n, const double* h_in, double* h_out, i
   }
 
   const int slot = eng == FFTOC_ENGINE_FX ? 1 : 0;
-  const int var = chosen_variant(slot, idx);
+  const int var = batch_variant(slot, idx, batch, nd.sms);
   const KernelDesc& d = nd.var[slot][idx].v[var];
   const void* tw = nd.twiddles + nd.tw_offset[slot][idx][var];
   const long long tiles = (batch + d.tpb - 1) / d.tpb;

@@ -126,9 +126,10 @@ inline cudaError_t fit_carveout(const void* fn, int threads, int smem, int* bloc
   return cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
 }
 
-// Dynamic shared memory of a launch on host buffers: more than half of an
-// SM's, so that one CTA runs per SM (launch_fwd_host).
-constexpr int kDirectSmem = 115 << 10;
+// Dynamic shared memory of a launch on host buffers, so large that `per_sm` CTAs
+// run per SM and no more (of its 228 KB, 1 KB of them the system's in each CTA).
+constexpr int direct_smem(int per_sm) { return (228 << 10) / (per_sm + 1) + 1024; }
+constexpr int kDirectSmem = direct_smem(1);
 // Dynamic shared-memory limit of a batched kernel: its own and that of its
 // launches on host buffers.  Every set-up of such a kernel sets this same
 // limit (the attribute belongs to the function, the last call wins).
@@ -172,11 +173,12 @@ fftoc_status launch_dmma(int n, const double* in, double* out, int64_t batch, cu
 
 // api.cu accessors: compiled plans per engine slot (0 F64, 1 FX), twiddle
 // tables of a plan (double2, or int32 limbs: build_twiddles), the plan
-// currently chosen for (slot, size index), AUTO resolution, and the
-// per-thread error message.
+// currently chosen for (slot, size index), the plan of a batch on a device of
+// `sms` SMs, AUTO resolution, and the per-thread error message.
 const SizeVariants* compiled_variants(int eng_slot);
 void twiddle_tables(const KernelDesc& d, std::vector<double>& f64, std::vector<int>& fx);
 int chosen_variant(int eng_slot, int idx);
+int batch_variant(int eng_slot, int idx, int64_t batch, int sms);
 int resolved_engine(int n, int engine);
 // The current device's twiddle table of plan (slot, size index, variant), its
 // error flag and SM count (device set-up on first use).

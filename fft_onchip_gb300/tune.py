@@ -35,10 +35,10 @@ def time_variants(n, engine, gib=0.5, reps=20, warmup=5, device=0, rounds=2):
     y = torch.empty_like(x)
     L = _lib.load()
     s = torch.cuda.current_stream()
-    cur = _lib.plan_query(n, eid)
+    before = _lib.plan_selected(n, eid)
     out = []
     try:
-        for v in range(cur["variants"]):
+        for v in range(_lib.plan_query(n, eid)["variants"]):
             _lib.plan_select(n, eid, v)
             for _ in range(warmup):
                 _lib.check(L.fftoc_c2c_fwd_ex(n, x.data_ptr(), y.data_ptr(), batch, eid, s.cuda_stream))
@@ -53,7 +53,7 @@ def time_variants(n, engine, gib=0.5, reps=20, warmup=5, device=0, rounds=2):
                 best = min(best, a.elapsed_time(b) / reps)
             out.append((v, best, _lib.plan_query(n, eid, variant=v)))
     finally:
-        _lib.plan_select(n, eid, cur["variant"])
+        _lib.plan_restore(n, eid, before)
     return out
 
 

@@ -147,7 +147,7 @@ fftoc_status fftoc_c2c_fwd_host(int n, const double *h_in, double *h_out, int64_
  * array compiled into the library (file-scope __device__ memory that every
  * GPU loading the library holds until exit): batch*n*16 must be at most
  * 32 MiB, larger batches are rejected with FFTOC_ERR_INVALID_VALUE.  H2D
- * copy, transform (the plan fftoc_plan_query reports) and D2H copy run on
+ * copy, transform (the plan fftoc_plan_query_batch reports) and D2H copy run on
  * `stream`; synchronise it before reading h_out.  All calls share that one
  * array: calls that overlap on the GPU (other streams, other host threads)
  * race and corrupt each other's results — serialise them.  The first call on
@@ -190,25 +190,34 @@ typedef struct {
 #define FFTOC_CODE_DIRECT_IO 8           /* small n: HBM accessed directly, no
                                             shared-memory staging of the tile */
 
-/* Plan currently used for (n, engine): the selected one, or while none was
- * selected variant 0 (the batched entry points then run batches of few
- * transforms on the plan noted at fftoc_plan_select). */
+/* Plan currently used for (n, engine): the selected one, or while none is
+ * selected variant 0, the plan of large batches (fftoc_plan_query_batch tells a
+ * smaller one's). */
 fftoc_status fftoc_plan_query(int n, int engine, fftoc_plan_info *info);
+
+/* Plan of a call on `batch` transforms on a device of `sms` multiprocessors:
+ * the selected one, or while none is selected the library's choice by the
+ * number of transforms per multiprocessor (few run on plans with shorter
+ * chains, whose results may differ in the last bits).  It holds for device and
+ * host buffers alike.  Needs no GPU. */
+fftoc_status fftoc_plan_query_batch(int n, int engine, int64_t batch, int sms, fftoc_plan_info *info);
 
 /* Any compiled plan of (n, engine), 0 <= variant < info.variants. */
 fftoc_status fftoc_plan_query_variant(int n, int engine, int variant, fftoc_plan_info *info);
 
 /* Use plan `variant` for (n, engine) from now on (process-wide), for every
- * batch.  While no plan is selected, the batched entry points on device memory
- * run batches of up to some number of transforms per SM (fixed point: 512 for
- * n = 8, 32 and 128, 128 for 16, 32 for 64, 256 for 256, 5 for 512, 3 for 1024,
- * 6 for 2048; binary64: 192 for 8, 48 for 16 and 32, 24 for 64, 12 for 128 and
- * 256, 7 for 512, 16 for 1024) on compiled plans with shorter chains, and larger
- * ones on variant 0.  The
+ * batch; variant 0 too, so a program that wants the library's choice back calls
+ * fftoc_plan_unselect.  The
  * reference picks executor parameters (UPB, FPU) at compile time through the
  * generated sweep, scripts/generate_bench.py:93-113; here the choice is made
  * at run time among the compiled plans. */
 fftoc_status fftoc_plan_select(int n, int engine, int variant);
+
+/* *variant = the selected plan of (n, engine), -1 while none is; and back to the
+ * library's choice.  To put a selection back after trying others: take
+ * fftoc_plan_selected first, then fftoc_plan_select it, or unselect for -1. */
+fftoc_status fftoc_plan_selected(int n, int engine, int *variant);
+fftoc_status fftoc_plan_unselect(int n, int engine);
 
 /* Autotuner: time every compiled plan of (n, engine) on a scratch batch of
  * `batch` transforms, select the fastest and return its index and time per

@@ -27,3 +27,15 @@ def cuda():
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     return torch
+
+
+@pytest.fixture(autouse=True)
+def plan_selections():
+    """Each test starts with the library's own choice of plans: a selection holds
+    for the rest of the process."""
+    yield
+    from fft_onchip_gb300 import _lib
+    if _lib._lib is not None:
+        for n in _lib.SIZES:
+            for engine in (_lib.ENGINE_F64, _lib.ENGINE_FX):
+                _lib.plan_restore(n, engine, None)
