@@ -290,11 +290,12 @@ constexpr bool EARLY_SMALL_TW = s == 1 && s == PL::S - 1 && PL::R[s] <= 4;
 template <class PL, int s>
 constexpr bool SUM_TW = s + 2 == PL::S && PL::R[s + 1 < PL::S ? s + 1 : s] == 2;
 
-// Limbs of -(wr + wi) = -(2 wr + (wi - wr)); |wr + wi| <= sqrt2 2^62.
-__device__ __forceinline__ int2 exact_tw_sum(const int4 w) {
+// Limbs of -(wr + wi) = -(wr + (wr + (wi - wr))), in this order: 2 wr of the
+// entry 1 is 2^63; |wi| <= 2^62, |wr + wi| <= sqrt2 2^62.
+FFTOC_HD int2 exact_tw_sum(const int4 w) {
   const long long r = ((long long)w.x << 32) + w.y, d = ((long long)w.z << 32) + w.w;
   int2 c;
-  EngFxN::split(-(2 * r + d), c.x, c.y);
+  EngFxN::split(-(r + (r + d)), c.x, c.y);
   return c;
 }
 
