@@ -29,6 +29,7 @@ ENGINES = {"auto": ENGINE_AUTO, "f64": ENGINE_F64, "fx": ENGINE_FX, "dmma": ENGI
 SPLIT_BF16X3, SPLIT_TF32X2, SPLIT_EXACT = 1, 2, 3
 
 SIZES = (8, 16, 32, 64, 128, 256, 512, 1024, 2048, 4096)
+EXEC_LAYOUT = 2  # FFTOC_EXEC_LAYOUT
 
 # Every symbol include/fftoc.h declares.
 EXPORTS = tuple(["fftoc_c2c_fwd_n%d" % n for n in SIZES]) + (
@@ -67,6 +68,7 @@ EXPORTS = tuple(["fftoc_c2c_fwd_n%d" % n for n in SIZES]) + (
     "fftoc_onchip_plan",
     "fftoc_onchip_run",
     "fftoc_selftest_bounded_wait",
+    "fftoc_exec_table",
     "fftoc_exec_twiddles",
 )
 
@@ -207,6 +209,8 @@ def load(path=None):
     L.fftoc_onchip_run.restype = c_int
     L.fftoc_selftest_bounded_wait.argtypes = [ctypes.c_double, vp]
     L.fftoc_selftest_bounded_wait.restype = c_int
+    L.fftoc_exec_table.argtypes = [c_int, c_int, ctypes.POINTER(c_int), c_int, ctypes.POINTER(vp)]
+    L.fftoc_exec_table.restype = c_int
     L.fftoc_exec_twiddles.argtypes = [c_int, c_int, ctypes.POINTER(c_int), ctypes.POINTER(vp)]
     L.fftoc_exec_twiddles.restype = c_int
     _lib = L

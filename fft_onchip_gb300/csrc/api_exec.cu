@@ -3,8 +3,10 @@
 // The executors are compiled into the caller's own kernels (the reference's
 // harness instantiates testing::fft_tester<CT, FFTExec, ...> itself,
 // includes/testing.cuh:16-57), so the library only supplies the tables: one
-// per (device, engine, radices), built with the same long-double twiddles as
-// the library's own plans and kept until the process exits.
+// per (device, engine, radices, layout), built with the same long-double
+// twiddles as the library's own plans and kept until the process exits.  The
+// layout is that of the header an executor was compiled with: an older object
+// asks for the older one and computes what it did.
 #include <array>
 #include <map>
 #include <mutex>
@@ -20,7 +22,7 @@ namespace {
 
 struct ExecTables {
   std::mutex mu;
-  std::map<std::array<int, 6>, void*> table;  // (device, engine slot, radices) -> device table
+  std::map<std::array<int, 7>, void*> table;  // (device, engine slot, layout, radices) -> device table
 };
 ExecTables g_exec;
 
@@ -30,6 +32,10 @@ bool radix_ok(int r) { return r == 2 || r == 4 || r == 8 || r == 16; }
 }  // namespace fftoc
 
 extern "C" fftoc_status fftoc_exec_twiddles(int n, int engine, const int radix[4], const void** table) {
+  return fftoc_exec_table(n, engine, radix, 1, table);
+}
+
+extern "C" fftoc_status fftoc_exec_table(int n, int engine, const int radix[4], int layout, const void** table) {
   using namespace fftoc;
   if (!table || !radix) return set_error(FFTOC_ERR_INVALID_VALUE, "null argument");
   *table = nullptr;
@@ -38,10 +44,12 @@ extern "C" fftoc_status fftoc_exec_twiddles(int n, int engine, const int radix[4
   const int eng = engine == FFTOC_ENGINE_AUTO ? FFTOC_ENGINE_FX : engine;
   if (eng != FFTOC_ENGINE_F64 && eng != FFTOC_ENGINE_FX)
     return set_error(FFTOC_ERR_UNSUPPORTED, "executors exist for the binary64 and fixed-point engines");
+  if (layout < 1 || layout > FFTOC_EXEC_LAYOUT)
+    return set_error(FFTOC_ERR_UNSUPPORTED, "executors compiled with a newer fftoc/exec.cuh than this library's");
 
   KernelDesc d;
-  d.natural = n >= kNaturalMinN ? 1 : 0;
-  d.tangent = eng == FFTOC_ENGINE_F64 ? 1 : 0;
+  d.natural = layout >= 2 && n >= kNaturalMinN ? 1 : 0;
+  d.tangent = layout >= 2 && eng == FFTOC_ENGINE_F64 ? 1 : 0;
   long long prod = 1;
   bool tail = false;  // an unused pass (1) was seen: only 1s may follow
   for (int s = 0; s < 4; ++s) {
@@ -65,7 +73,7 @@ extern "C" fftoc_status fftoc_exec_twiddles(int n, int engine, const int radix[4
     cudaGetLastError();
     return set_error(FFTOC_ERR_CUDA, std::string("cudaGetDevice: ") + cudaGetErrorString(e));
   }
-  const std::array<int, 6> key = {dev, eng, d.radix[0], d.radix[1], d.radix[2], d.radix[3]};
+  const std::array<int, 7> key = {dev, eng, layout, d.radix[0], d.radix[1], d.radix[2], d.radix[3]};
   std::lock_guard<std::mutex> lock(g_exec.mu);
   auto it = g_exec.table.find(key);
   if (it != g_exec.table.end()) {

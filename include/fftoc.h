@@ -44,7 +44,7 @@
 extern "C" {
 #endif
 
-#define FFTOC_VERSION 10000 /* 1.0.0 */
+#define FFTOC_VERSION 10100 /* 1.1.0 */
 
 typedef enum {
   FFTOC_OK = 0,
@@ -364,13 +364,18 @@ fftoc_status fftoc_onchip_run(int n, int engine, double *data, int64_t blocks, i
 /* Twiddle table for the device-side executors of <fftoc/exec.cuh> (the
  * FFTExec shape of includes/tensor_fft_64.cuh:12-45): the table of a plan of
  * size n whose passes have radices radix[0..3] (each 2, 4, 8 or 16, unused
- * passes 1 at the end), in the engine's layout (binary64, 16 bytes per entry,
- * or fixed-point limbs, 16 bytes for n <= 32 and 24 from 64 up: the layout
- * belongs to the <fftoc/exec.cuh> shipped with the library, so compile
- * executors against the header of the library they run with), in device memory
- * of the current device owned by the library until the process exits.  *table is NULL for a
+ * passes 1 at the end), in the engine's layout, in device memory of the current
+ * device owned by the library until the process exits.  *table is NULL for a
  * one-pass plan (no twiddles).  Engines: binary64, fixed point (AUTO
- * resolves to the latter).  Synchronous on first use of a plan. */
+ * resolves to the latter).  Synchronous on first use of a plan.
+ * `layout` is the FFTOC_EXEC_LAYOUT that the executors were compiled with:
+ *   1  binary64 (cos, -sin), or four 30-bit limbs: 16 bytes an entry
+ *   2  binary64 with tangent forms; fixed point from n = 64 up on natural words,
+ *      24 bytes an entry
+ * A layout that the library does not know is FFTOC_ERR_UNSUPPORTED.
+ * fftoc_exec_twiddles is layout 1, which headers before version 1.1 expect. */
+#define FFTOC_EXEC_LAYOUT 2
+fftoc_status fftoc_exec_table(int n, int engine, const int radix[4], int layout, const void **table);
 fftoc_status fftoc_exec_twiddles(int n, int engine, const int radix[4], const void **table);
 
 /* Device-side error flags of the current device, those of every entry point

@@ -25,7 +25,7 @@
 // the tile doubles as the exchange area between passes.  Arithmetic, plans
 // and error bounds are the library's (relative L2 error ~1e-15 for the
 // fixed-point engine).  Twiddle tables live in device memory owned by
-// libfftoc (fftoc_exec_twiddles); bind() copies their addresses into this
+// libfftoc (fftoc_exec_table); bind() copies their addresses into this
 // translation unit.  An executor whose table is not bound writes quiet NaNs
 // instead of transforming (sizes with one pass need no table).
 #pragma once
@@ -208,8 +208,8 @@ template <int N>
 inline fftoc_status bind_size(const void* (&h)[2][kSizes]) {
   using PL = typename plan_of<N, 1>::type;
   const int radix[4] = {PL::R[0], PL::R[1], PL::R[2], PL::R[3]};
-  fftoc_status st = fftoc_exec_twiddles(N, FFTOC_ENGINE_F64, radix, &h[0][size_slot(N)]);
-  if (st == FFTOC_OK) st = fftoc_exec_twiddles(N, FFTOC_ENGINE_FX, radix, &h[1][size_slot(N)]);
+  fftoc_status st = fftoc_exec_table(N, FFTOC_ENGINE_F64, radix, FFTOC_EXEC_LAYOUT, &h[0][size_slot(N)]);
+  if (st == FFTOC_OK) st = fftoc_exec_table(N, FFTOC_ENGINE_FX, radix, FFTOC_EXEC_LAYOUT, &h[1][size_slot(N)]);
   return st;
 }
 template <int... Ns>

@@ -43,7 +43,7 @@ template __global__ void testing::fft_tester<CT, L256, 256, L256::units_per_bloc
 
 // What fftoc::exec::bind() does from host code of an executor's own
 // translation unit: store the twiddle-table addresses (from
-// fftoc_exec_twiddles) in this module's table, [engine][size slot].
+// fftoc_exec_table) in this module's table, [engine][size slot].
 extern "C" __global__ void fftoc_harness_bind(const void* const* tables) {
   const int i = threadIdx.x;
   if (i < 2 * fftoc::exec::kSizes) fftoc::exec::g_tables[i / fftoc::exec::kSizes][i % fftoc::exec::kSizes] = tables[i];

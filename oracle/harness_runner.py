@@ -6,7 +6,7 @@ testing::fft_tester, the kernel of the reference's own harness
 (includes/testing.cuh:16-57), compiled unmodified and instantiated with this
 library's executors under the reference's names (include/fftoc/compat.cuh).
 This module loads it with the CUDA driver API, binds the executors to the
-library's twiddle tables (fftoc_exec_twiddles, as fftoc::exec::bind() does)
+library's twiddle tables (fftoc_exec_table, as fftoc::exec::bind() does)
 and launches it with the geometry of the reference's host driver
 run_fft_kernel (includes/testing.cuh:59-92): block (Exec::threads,
 Exec::units_per_block), shared memory 16 * Size * units_per_block *
@@ -15,6 +15,8 @@ ffts_per_unit bytes, arguments (inner_repeats, data, with_transfers).
 import ctypes
 import json
 import os
+
+from fft_onchip_gb300 import _lib
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CUBIN = os.path.join(HERE, "_ref", "harness_kernels.cubin")
@@ -86,9 +88,9 @@ class Harness:
             for i, n in enumerate(SIZES):
                 r = RADICES[n] + [1] * (4 - len(RADICES[n]))
                 out = ctypes.c_void_p()
-                st = lib.fftoc_exec_twiddles(n, e, (ctypes.c_int * 4)(*r), ctypes.byref(out))
+                st = lib.fftoc_exec_table(n, e, (ctypes.c_int * 4)(*r), _lib.EXEC_LAYOUT, ctypes.byref(out))
                 if st != 0:
-                    raise RuntimeError("fftoc_exec_twiddles(%d) = %d" % (n, st))
+                    raise RuntimeError("fftoc_exec_table(%d) = %d" % (n, st))
                 ptrs[slot * 10 + i] = out.value or 0
         d = t.tensor(ptrs, dtype=t.int64, device="cuda")
         self._launch(self._fn("fftoc_harness_bind"), 1, (32, 1), 0, [ctypes.c_uint64(d.data_ptr())])
