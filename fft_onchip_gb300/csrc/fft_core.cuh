@@ -636,7 +636,8 @@ FFTOC_HD void fxn_dft16(long long (&re)[PP], long long (&im)[PP]) {
 // transforms of 256 points 195 -> 174 us, 64 MiB of 64 to 4096 points 9 to 12 %
 // less time; errors against long double are 2 to 4 % smaller at every size.
 // Inside, values reach sqrt(2) times those of the plain products, as they do
-// in W8 = H (1 - j).  The step takes the
+// in W8 = H (1 - j): transforms that this could make overflow are scaled
+// (F64Range).  The step takes the
 // sums a_m at B + m ST and differences b_m at B + (m + R/2) ST, m < R/2, to
 // the R outputs in natural order.
 template <int R, int B, int ST, int PP>

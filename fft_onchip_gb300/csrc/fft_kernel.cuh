@@ -341,7 +341,65 @@ __device__ __forceinline__ int fx_transform_max(int em, int tid, int j, int* red
   return em;
 }
 
-// Programmatic dependent launch (launch_plan): a kernel may start while the one
+// Binary64 transforms with a component of 2^1021 / N or more: the outputs are
+// below 2 N times the largest component, and inside EngF64's butterflies values
+// reach sqrt(2) times the moduli of the plain products, which may overflow where
+// no output does.  Such transforms (non-finite ones with them) run on inputs
+// scaled by 2^-down, and their outputs are scaled back: both exact but for
+// outputs that are not representable, and for parts 2^-1000 times the largest.
+template <int N> struct F64Range {
+  static constexpr int down = ilog2c(N) + 4;
+  // the largest exponent field that is transformed as it is: all below 2^1021 / N,
+  // and below the fields that f64_exponent cannot tell apart
+  static constexpr int top = 2044 - ilog2c(N) < 2039 ? 2044 - ilog2c(N) : 2039;
+};
+// The largest exponent field of a thread's points, ordered as binary32 values
+// (fx_exponent_range); 0x7F8 or 0x7FF for fields from 0x7F8 up.
+template <int P>
+__device__ __forceinline__ int f64_exponent(const double (&re)[P], const double (&im)[P]) {
+  float m = 0.0f;
+#pragma unroll
+  for (int i = 0; i < P; ++i) {
+    const float a = fabsf(__int_as_float(__double2hiint(re[i]))), b = fabsf(__int_as_float(__double2hiint(im[i])));
+    asm("max.NaN.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(a), "f"(b));
+  }
+  return (int)(__float_as_uint(m) >> 20);
+}
+// Values times 2^-D and back, on the words: predicated multiplications would
+// occupy the FP64 pipe in every transform (38 % more time at N = 16).  Infinities
+// and NaNs stay, values below 2^(D - 1022) become zero, and on the way back what
+// is not representable becomes an infinity.
+template <int D>
+__device__ __forceinline__ double f64_down(double v) {
+  const int hi = __double2hiint(v), a = hi & 0x7FFFFFFF;
+  const bool none = a < ((D + 1) << 20);
+  return __hiloint2double(none ? 0 : a >= 0x7FF00000 ? hi : hi - (D << 20), none ? 0 : __double2loint(v));
+}
+template <int D>
+__device__ __forceinline__ double f64_up(double v) {
+  const int hi = __double2hiint(v), a = hi & 0x7FFFFFFF;
+  if (a < (1 << 20) || a >= 0x7FF00000) return v;
+  const bool over = a >= ((0x7FF - D) << 20);
+  return __hiloint2double(over ? (hi & (int)0x80000000) | 0x7FF00000 : hi + (D << 20), over ? 0 : __double2loint(v));
+}
+template <int D, int P>
+__device__ __forceinline__ void f64_scale_down(double (&re)[P], double (&im)[P]) {
+#pragma unroll
+  for (int i = 0; i < P; ++i) {
+    re[i] = f64_down<D>(re[i]);
+    im[i] = f64_down<D>(im[i]);
+  }
+}
+template <int D, int P>
+__device__ __forceinline__ void f64_scale_up(double (&re)[P], double (&im)[P]) {
+#pragma unroll
+  for (int i = 0; i < P; ++i) {
+    re[i] = f64_up<D>(re[i]);
+    im[i] = f64_up<D>(im[i]);
+  }
+}
+
+// Programmatic dependent launch (launch_overlapped): a kernel may start while the one
 // before it in its stream drains.  after_previous() waits for that kernel's
 // completion and must come before any access to the caller's buffers;
 // allow_next(), after it, lets the next kernel's CTAs take the places that this
@@ -368,6 +426,13 @@ __device__ __forceinline__ double2 load_point(const double2* p) {
   double2 v;
   asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
   return v;
+}
+
+// A store without a branch, which would keep the stores behind the last pass.
+__device__ __forceinline__ void store_point_if(double2* p, double2 v, bool on) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %3, 0;\n\t@q st.global.v2.f64 [%0], {%1, %2};\n\t}" ::"l"(p), "d"(v.x),
+               "d"(v.y), "r"((int)on)
+               : "memory");
 }
 
 // --- the kernel ---------------------------------------------------------------
@@ -518,12 +583,56 @@ struct Fft {
       run_passes<s + 1>(re, im, j, t, tw, sm);
     }
   }
+
+  // The passes of the CTA's binary64 transforms.  True if one of them may
+  // overflow on the way (F64Range, on the first pass's outputs); then no output
+  // is stored, and redo_ranged() follows.  The vote is the first exchange's
+  // barrier, and nothing branches on it before the stores: a branch there keeps
+  // the next pass's twiddle loads from moving above the barrier (N = 512 to 4096,
+  // one transform: 2 to 6 % more time).
+  __device__ __forceinline__ static bool run_voted(double (&re)[P], double (&im)[P], bool check, int j, int t,
+                                                   const TW* __restrict__ tw, longlong2* sm) {
+    pass<0>(re, im, t, tw, std::make_integer_sequence<int, P / PL::R[0]>{});
+    const bool large = check && f64_exponent(re, im) > F64Range<N / PL::R[0]>::top;
+    write_smem<0>(re, im, j, t, sm);
+    const bool hold = __syncthreads_or(large);
+    read_smem(re, im, j, t, sm);
+    run_passes<1>(re, im, j, t, tw, sm);
+    return hold;
+  }
+
+  // The CTA's transforms again from their inputs, those of large values scaled;
+  // src and dst are this thread's transform.  Out of line: inlined it took the
+  // kernels' registers (binary64, 1,500 transforms of 256 points 17.7 -> 20.6 us).
+  __device__ __noinline__ static void redo_ranged(const double2* src, double2* dst, bool active, const TW* tw,
+                                                  longlong2* sm, int* red) {
+    const int tid = threadIdx.x, j = tid / T, t = tid - j * T;
+    double re[P], im[P];
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      const double2 v = active ? src[t + T * i] : make_double2(0.0, 0.0);
+      re[i] = v.x;
+      im[i] = v.y;
+    }
+    __syncthreads();  // the last readers of the exchange buffer and of `red` are done
+    const bool scaled = fx_transform_max<T, TPB>(f64_exponent(re, im), tid, j, red) > F64Range<N>::top;
+    if (scaled) f64_scale_down<F64Range<N>::down>(re, im);
+    run_passes<0>(re, im, j, t, tw, sm);
+    if (scaled) f64_scale_up<F64Range<N>::down>(re, im);
+    if (!active) return;
+    constexpr int RL = PL::R[NS - 1], BL = P / RL;
+#pragma unroll
+    for (int b = 0; b < BL; ++b)
+#pragma unroll
+      for (int m = 0; m < RL; ++m) dst[dest<NS - 1>(t, b, m)] = make_double2(re[b + BL * m], im[b + BL * m]);
+  }
 };
 
 // Where the transforms of one CTA tile live.  IndexedTile (the uneven-batch
 // kernel): transform j of the tile at element base[j], with the bases staged in
 // shared memory by the caller.
 struct IndexedTile {
+  static constexpr bool REPEATS = false;
   const double2* __restrict__ in;
   double2* __restrict__ out;
   const long long* base;  // shared memory, one entry per transform of the tile
@@ -539,6 +648,7 @@ struct IndexedTile {
 // thread touches only its own transform): the thread's transform offset in a
 // register, loaded ahead by the caller.
 struct RegTile {
+  static constexpr bool REPEATS = false;
   const double2* __restrict__ in;
   double2* __restrict__ out;
   long long off;  // this thread's transform
@@ -555,6 +665,7 @@ struct RegTile {
 // shared loads.
 template <int N>
 struct SmemTile {
+  static constexpr bool REPEATS = true;  // outputs are inputs again, up to infinities
   double2* buf;
   long long tile0, count;  // tile0 = 0, count = TPB
   __device__ __forceinline__ const double2* in_of(int j) const { return buf + j * N; }
@@ -627,7 +738,25 @@ __device__ __forceinline__ void fft_tile(const Tile& tl, const typename E::TW* _
   }
 
   if constexpr (F::STAGED) __syncthreads();  // staging buffer is reused by the passes
-  F::template run_passes<0>(re, im, j, t, tw, sm);
+  // binary64: a transform of the CTA has to be redone (nothing is stored before);
+  // a transform that one thread holds is scaled where it is
+  bool hold = false, scaled = false, check = active;
+  if constexpr (E::kId == EngF64::kId && Tile::REPEATS) {  // scaling does nothing for infinities and NaNs
+#pragma unroll
+    for (int i = 0; i < P; ++i) check = check && expo_of(hi_word(re[i])) < 0x7FF && expo_of(hi_word(im[i])) < 0x7FF;
+  }
+  if constexpr (E::kId == EngF64::kId && NS > 1) {
+    hold = F::run_voted(re, im, check, j, t, tw, sm);
+  } else {
+    if constexpr (E::kId == EngF64::kId) {
+      scaled = check && f64_exponent(re, im) > F64Range<N>::top;
+      if (scaled) f64_scale_down<F64Range<N>::down>(re, im);
+    }
+    F::template run_passes<0>(re, im, j, t, tw, sm);
+    if constexpr (E::kId == EngF64::kId) {
+      if (scaled) f64_scale_up<F64Range<N>::down>(re, im);
+    }
+  }
 
   // ---- store: output m of butterfly b of the last pass is element dest(...)
   constexpr int RL = PL::R[NS - 1];
@@ -686,13 +815,13 @@ __device__ __forceinline__ void fft_tile(const Tile& tl, const typename E::TW* _
             make_longlong2(__double_as_longlong(v.x), __double_as_longlong(v.y));
       }
     __syncthreads();
-    for (int idx = tid; idx < tile_elems; idx += F::THREADS) {
+    for (int idx = tid; idx < (hold ? 0 : tile_elems); idx += F::THREADS) {
       const int jj = idx / N, e = idx - jj * N;
       const longlong2 v = sm[F::slot(jj, e)];
       *tl.out_elem(idx, jj, e) = make_double2(__longlong_as_double(v.x), __longlong_as_double(v.y));
     }
   } else {
-    if (active) {
+    if (active && !hold) {
       double2* dst = tl.out_of(j);
       if constexpr (FxTrunc<N>::value) {
 #pragma unroll
@@ -714,6 +843,9 @@ __device__ __forceinline__ void fft_tile(const Tile& tl, const typename E::TW* _
           for (int m = 0; m < RL; ++m) dst[F::template dest<NS - 1>(t, b, m)] = slow_value(b + BL * m);
       }
     }
+  }
+  if constexpr (E::kId == EngF64::kId && NS > 1) {
+    if (hold) F::redo_ranged(tl.in_of(j), tl.out_of(j), active, tw, sm, reinterpret_cast<int*>(smem_raw + TPB * F::NP * 16));
   }
 }
 
@@ -815,7 +947,21 @@ fft_fwd_kernel(const double2* __restrict__ in, double2* __restrict__ out, long l
   }
 
   if constexpr (F::STAGED) __syncthreads();  // staging buffer is reused by the passes
-  F::template run_passes<0>(re, im, j, t, tw, sm);
+  // binary64: a transform of the CTA has to be redone (nothing is stored before);
+  // a transform that one thread holds is scaled where it is
+  bool hold = false, scaled = false;
+  if constexpr (E::kId == EngF64::kId && NS > 1) {
+    hold = F::run_voted(re, im, active, j, t, tw, sm);
+  } else {
+    if constexpr (E::kId == EngF64::kId) {
+      scaled = f64_exponent(re, im) > F64Range<N>::top;
+      if (scaled) f64_scale_down<F64Range<N>::down>(re, im);
+    }
+    F::template run_passes<0>(re, im, j, t, tw, sm);
+    if constexpr (E::kId == EngF64::kId) {
+      if (scaled) f64_scale_up<F64Range<N>::down>(re, im);
+    }
+  }
 
   // ---- store: output m of butterfly b of the last pass is element dest(...)
   constexpr int RL = PL::R[NS - 1];
@@ -875,13 +1021,13 @@ fft_fwd_kernel(const double2* __restrict__ in, double2* __restrict__ out, long l
       }
     __syncthreads();
     double2* dst = out + tile0 * N;
-    for (int idx = tid; idx < tile_elems; idx += F::THREADS) {
+    for (int idx = tid; idx < (hold ? 0 : tile_elems); idx += F::THREADS) {
       const int jj = idx / N, e = idx - jj * N;
       const longlong2 v = sm[F::slot(jj, e)];
       dst[idx] = make_double2(__longlong_as_double(v.x), __longlong_as_double(v.y));
     }
   } else {
-    if (active) {
+    if (TPB == 1 ? active : active && !hold) {
       double2* dst = out + tr * N;
       if constexpr (FxTrunc<N>::value) {
 #pragma unroll
@@ -894,7 +1040,9 @@ fft_fwd_kernel(const double2* __restrict__ in, double2* __restrict__ out, long l
         for (int b = 0; b < BL; ++b) {
           double2* q = dst + F::template dest<NS - 1>(t, b, 0);
 #pragma unroll
-          for (int m = 0; m < RL; ++m) q[m * PL::span(NS - 1)] = value(b + BL * m);
+          for (int m = 0; m < RL; ++m)
+            if constexpr (E::kId == EngF64::kId && TPB == 1) store_point_if(q + m * PL::span(NS - 1), value(b + BL * m), !hold);
+            else q[m * PL::span(NS - 1)] = value(b + BL * m);
         }
       } else {
 #pragma unroll
@@ -903,6 +1051,9 @@ fft_fwd_kernel(const double2* __restrict__ in, double2* __restrict__ out, long l
           for (int m = 0; m < RL; ++m) dst[F::template dest<NS - 1>(t, b, m)] = slow_value(b + BL * m);
       }
     }
+  }
+  if constexpr (E::kId == EngF64::kId && NS > 1) {
+    if (hold) F::redo_ranged(in + tr * N, out + tr * N, active, tw, sm, reinterpret_cast<int*>(smem_raw + TPB * F::NP * 16));
   }
 }
 

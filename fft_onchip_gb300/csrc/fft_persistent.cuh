@@ -172,14 +172,16 @@ fft_fwd_persistent(const double2* __restrict__ in, double2* __restrict__ out, lo
       fx_convert_in<P, false, TR>(raw, re, im, sc.eref, emin);
     }
     if constexpr (NS > 1) __syncthreads();  // every linear read is done before pass-0 writes
-    F::template run_passes<0>(re, im, j, t, tw, sm);
+    bool hold = false;  // binary64: a transform of the CTA has to be redone
+    if constexpr (E::kId == EngF64::kId) hold = F::run_voted(re, im, active, j, t, tw, sm);
+    else F::template run_passes<0>(re, im, j, t, tw, sm);
 
     // fixed point: one branch per thread between the fast conversion and, for
     // the rare transforms whose outputs leave the normal range (or had
     // non-finite inputs), the slow one
     constexpr int RL = PL::R[NS - 1];
     constexpr int BL = P / RL;
-    if (active) {
+    if (active && !hold) {
       double2* dst = out + tr * N;
       if (E::kId == EngF64::kId || !(slow || special)) {
 #pragma unroll
@@ -207,6 +209,9 @@ fft_fwd_persistent(const double2* __restrict__ in, double2* __restrict__ out, lo
                         : make_double2(fx_out_slow((long long)re[i], K), fx_out_slow((long long)im[i], K));
           }
       }
+    }
+    if constexpr (E::kId == EngF64::kId) {
+      if (hold) F::redo_ranged(in + tr * N, out + tr * N, active, tw, sm, red);
     }
     // this thread's generic-proxy writes to stage s are ordered before the
     // bulk copy that refills it (async proxy) after the barrier

@@ -110,13 +110,15 @@ struct fft {
 
     S re[P], im[P];
     int K = 0, kshift = 0;
-    bool slow = false, special = false;
+    bool slow = false, special = false, scaled = false;
+    __shared__ int red[transforms_per_block * (T > 32 ? T / 32 : 1)];
     if constexpr (E::kId == EngF64::kId) {
 #pragma unroll
       for (int i = 0; i < P; ++i) { re[i] = raw[i].x; im[i] = raw[i].y; }
+      scaled = fx_transform_max<T, transforms_per_block>(f64_exponent(re, im), tid, j, red) > F64Range<Size>::top;
+      if (scaled) f64_scale_down<F64Range<Size>::down>(re, im);
     } else {
       // largest biased exponent of the transform, smallest of this thread
-      __shared__ int red[transforms_per_block * (T > 32 ? T / 32 : 1)];
       constexpr bool TR = FxTrunc<Size>::value;
       int em, emin;
       fx_exponent_range<P, TR>(raw, em, emin);
@@ -140,6 +142,9 @@ struct fft {
       return;
     }
     run<0>(re, im, j, t, tw, sm);
+    if constexpr (E::kId == EngF64::kId) {
+      if (scaled) f64_scale_up<F64Range<Size>::down>(re, im);
+    }
     if constexpr (NS > 1) __syncthreads();  // every thread has read its last exchange
 
     if constexpr (E::kId == EngF64::kId) {
