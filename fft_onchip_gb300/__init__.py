@@ -40,13 +40,14 @@ _size_entry = {}
 def fft_ptr(n, in_ptr, out_ptr, batch, stream_ptr=0, engine="auto"):
     """Raw C-ABI call: device pointers, batch count, cudaStream_t as int."""
     if engine == "auto" or (not isinstance(engine, str) and int(engine) == ENGINE_AUTO):
+        n = int(n)
         fn = _size_entry.get(n)
         if fn is None and n in SIZES:
-            fn = _size_entry[int(n)] = getattr(load(), "fftoc_c2c_fwd_n%d" % n)
+            fn = _size_entry[n] = getattr(load(), "fftoc_c2c_fwd_n%d" % n)
         if fn is not None:
             status = fn(in_ptr, out_ptr, int(batch), stream_ptr)
             return status if status == 0 else check(status)
-        return check(load().fftoc_c2c_fwd(int(n), in_ptr, out_ptr, int(batch), stream_ptr))
+        return check(load().fftoc_c2c_fwd(n, in_ptr, out_ptr, int(batch), stream_ptr))
     return check(load().fftoc_c2c_fwd_ex(int(n), in_ptr, out_ptr, int(batch), _engine_id(engine), stream_ptr))
 
 
