@@ -90,7 +90,8 @@ struct EngF64 {
     xr = r;
     xi = i;
   }
-  // The tangent form of w = c + j s: w x = a y with y two multiply-adds,
+  // The tangent form of w = c + j s (the FFT for fused multiply-add machines of
+  // Linzer and Feig, 1993): w x = a y with y two multiply-adds,
   //   |s| <= |c|: a = c, b = s / c,  y = x + j b x,
   //   else:       a = s, b = -c / s, y = j x + j b (j x),
   // and A + w x, A - w x then four more: a radix-2 butterfly in 6 instructions

@@ -44,13 +44,14 @@
 // 8h..8h+7, writes their A digits and reads its 16 accumulator columns of
 // each order.
 //
-// Bound by latency and by the integer pipes (both 35 to 45 % busy, 16 warps per
-// SM, the limit of the registers and of the exchange buffers).  Products on
+// No pipe is above 45 % busy, issue slots 46 %, at 16 warps per SM, the limit of
+// the registers and of the exchange buffers; 32 warps (four threads a row)
+// issued only 7 % more, so which wait bounds it is not known.  Products on
 // the natural 32-bit words at quarter scale instead of 30-bit limbs, one
 // binary32-ordered exponent range for the maximum and the fast-path test, and
 // the combination of the slices in two instructions less took 2^26 points from
-// 687, 641, 649, 791, 897, 936, 963 and 1380 us (N = 32 to 4096) to 627, 619,
-// 629, 755, 853, 883, 900 and 1348 us.
+// 687, 641, 649, 791, 897, 936, 963 and 1380 us (N = 32 to 4096) to 628, 618,
+// 596, 759, 852, 882, 901 and 1348 us.
 #pragma once
 #include <cuda_fp16.h>
 

@@ -145,8 +145,13 @@ inline cudaError_t allow_shared(const void* fn, int smem) {
 // `wave` is the number of CTAs that fit the device at once.  A grid of 1/2 to
 // 2/3 of it is launched without the overlap: two such grids do not fit
 // together, so the next one's CTAs crowd on some SMs, and back to back that
-// measured up to 14 % slower at N = 256, 512, 1024 and 2048 (7-15 % faster at
-// 64, 128 and 4096); below and above the overlap wins at every N, by 3-70 %.
+// measured up to 14 % slower for the fixed-point plans of N = 256, 512, 1024 and
+// 2048 (7-15 % faster at 64, 128 and 4096); below and above the overlap wins at
+// every N, by 3-70 %.  The rule goes by the grid alone.  Where it keeps such grids
+// of the split kernels and of host buffers from the overlap, they would gain:
+// BF16x3 and the exact slices 10 to 30 % (512 points 10.3 against 8.1 us and
+// 14.4 against 11.0), TF32x2 at N = 16 and 4096 as much, host buffers 5 to 20 %
+// up to N = 1024 and -3 to 4 % above.
 inline cudaError_t launch_overlapped(const void* fn, unsigned blocks, long long wave, int threads, int smem,
                                      void** args, cudaStream_t stream, bool overlap = true) {
   cudaLaunchConfig_t cfg = {};
