@@ -82,3 +82,18 @@ def test_other_entry_points(cuda, fftoc_lib):
         d = cuda.from_numpy(x).cuda()
         _lib.check(fftoc_lib.fftoc_onchip_run(n, F.ENGINE_F64, d.data_ptr(), 1, 1, cuda.cuda.current_stream().cuda_stream))
         check(d.cpu().numpy(), x)
+
+
+@pytest.mark.parametrize("n", _lib.SIZES)
+def test_in_place(cuda, fftoc_lib, n):
+    """Tiles that are redone read their inputs again: nothing of them is stored before."""
+    import fft_onchip_gb300 as F
+    x = large_rows(n)
+    x = np.concatenate([x, inputs.normal(n, len(x) // 2, seed=n), x[::-1]])
+    for v in range(F.plan_query(n, F.ENGINE_F64)["variants"]):
+        F.plan_select(n, F.ENGINE_F64, v)
+        d = cuda.from_numpy(x).cuda()
+        want = F.fft(d, engine="f64")
+        F.fft(d, out=d, engine="f64")
+        assert cuda.equal(cuda.view_as_real(d), cuda.view_as_real(want)), v
+        check(d.cpu().numpy(), x)
